@@ -24,8 +24,10 @@
 #include "../../include/qgrad.h"
 #include "qg_batched.h"
 #include "qg_extra.h"
+#include "qg_fixed.h"
 #include "qg_internal.cuh"
 #include "qg_kernels.h"
+#include "qg_ladder.cuh"
 #include "qg_shots.h"
 
 using namespace qg;
@@ -271,25 +273,211 @@ int build_layer(int n, const Layout& lay, const std::vector<LayerGate>& g, int8_
   return QG_OK;
 }
 
+// ------------------------------------------------------------ fixed-point sweeps (qg_fixed.cu)
+
+// complex128 circuits run on the fixed-point sweeps wherever those have an
+// instantiation: from 9 qubits on (below, a state is one tile of the double
+// kernels either way), tiles of 9..12 bits, an integer cost, and unless the
+// single-buffered double kernels are asked for.
+bool fixed_path(const qg_circuit* c, int dtype) {
+  if (dtype != QG_C128 || c->n < FIX_TMIN || c->L < 1) return false;
+  if (c->kind == 1 && c->cost_kind != COST_INT) return false;
+  const int t = c->tune_tile_bits[0];
+  if (t != 0 && (t < FIX_TMIN || t > FIX_TMAX)) return false;
+  return fwd_pipelined(c, dtype);
+}
+
+struct FixSweep {
+  int t, lo, k;  // tile bits, lowest active bit, active bits
+};
+
+// Sweeps of one layer: A = bits [0, t), then the high bits, each tile padded
+// with the lowest bits.  A tuned size holds for every tile.  The default,
+// measured per grad_run (ms, L = 20 unless said; t:k per sweep):
+//  - n <= 11: one sweep of one tile (n = 11: 0.60 against 0.63 for 9:9,9:2;
+//    n = 12: 0.94 against 0.66, so two from there on).
+//  - Small states leave SMs idle: the smallest tiles that need two sweeps
+//    (n = 16: 9:9,9:7 0.79, 10:10,10:6 0.83; n = 18: 10:10,10:8 1.07,
+//    9:9,9:9 1.31, 12:12,12:6 1.62; n = 19: 12:12,12:7 1.77, 11:11,11:8
+//    1.91, 10:10,10:9 1.96).
+//  - n = 20, 21 stay in L2, where runs shorter than 128 bytes cost nothing:
+//    two sweeps of 11-bit tiles (n = 20: 2.42; 12:12,12:8 2.62;
+//    10:10,10:5,10:5 2.78).
+//  - From 22 on three sweeps (four from 31), 128-byte runs, and 10-bit tiles
+//    where they suffice (n = 24, L = 10: 14.3; 11:11,11:8,11:5 15.6;
+//    9:9,9:6,9:6,9:3 14.9).  From n = 28 four sweeps of 10-bit tiles are
+//    faster than three of 11- and 12-bit ones (n = 28, L = 2 uncompute:
+//    65.7; 12:12,11:8,11:8 70.4), but a history would hold a third more
+//    states, so that form keeps three.
+std::vector<FixSweep> fix_layout(int n, int tile_bits, bool history) {
+  std::vector<FixSweep> out;
+  auto rest = [&](int lo, int sweeps, int t) {  // the high bits over so many sweeps
+    for (int s = sweeps; s > 0; --s) {
+      const int k = (n - lo + s - 1) / s;
+      out.push_back({t > 0 ? t : k <= 7 ? 10 : k + 3, lo, k});
+      lo += k;
+    }
+  };
+  if (tile_bits > 0) {
+    const int t = std::min(n, tile_bits);
+    out.push_back({t, 0, t});
+    for (int lo = t; lo < n;) {
+      const int k = std::min(t - 3, n - lo);
+      out.push_back({t, lo, k});
+      lo += k;
+    }
+    return out;
+  }
+  if (n <= 21) {
+    const int t = n <= 11 ? n : n <= 16 ? 9 : n <= 18 ? 10 : n == 19 ? 12 : 11;
+    out.push_back({t, 0, t});
+    if (t < n) rest(t, 1, t);
+    return out;
+  }
+  const int high = n >= 31 || (n >= 28 && !history) ? 3 : 2;
+  const int choice[][2] = {{10, 7}, {11, 7}, {11, 8}, {12, 8}, {12, 9}};
+  for (const auto& ch : choice)
+    if (n - ch[0] <= high * ch[1]) {
+      out.push_back({ch[0], 0, ch[0]});
+      rest(ch[0], high, 0);
+      return out;
+    }
+  out.push_back({12, 0, 12});
+  rest(12, (n - 12 + 8) / 9, 12);
+  return out;
+}
+
 struct Program {
   Layout lay;
   std::vector<SweepDesc> sweeps;
+  bool fixed = false;          // the fixed-point sweeps run this circuit (fix instead of sweeps)
+  std::vector<FixDesc> fix;
+  FixTables ft;
+  size_t area_bytes = 0;       // their phase tables
   int8_t obs_pre = ENT_NONE;  // entangler between the last sweep and the observable
   int8_t periodic = 0;        // the CNOT ladder is the periodic one
   int first_param = 0;   // first sweep with gradient slots
   int nslots = 0;        // gradient slots (before the expectation slots)
   int grad_kind = 0;     // finalize layout
   int nparams = 0;
+  int nsweeps() const { return (int)(fixed ? fix.size() : sweeps.size()); }
+  int8_t pre(int k) const { return fixed ? fix[k].pre : sweeps[k].pre; }
 };
 
-int build_program(const qg_circuit* c, int dtype, bool with_ini, Program& P) {
+int8_t ent_of(const qg_circuit* c) {
+  return (c->entangler == QG_ENT_CNOT_LADDER || c->entangler == QG_ENT_CNOT_LADDER_PERIODIC) ? ENT_CNOT
+         : c->entangler == QG_ENT_CZ_LADDER                                          ? ENT_CZ
+                                                                                     : ENT_NONE;
+}
+
+// The fixed-point sweeps of a circuit: per layer one descriptor per sweep,
+// with every rotation in the sweep that owns its bit.
+void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
+  const int n = c->n;
+  const std::vector<FixSweep> lay = fix_layout(n, c->tune_tile_bits[0], op == QG_OP_GRAD_HISTORY);
+  const int per = (int)lay.size();
+  const bool mc = c->kind == 0;
+  const int ini = mc && with_ini ? 1 : 0;
+  const int layers = c->L + ini;
+  FixTables& f = P.ft;
+  memset(&f, 0, sizeof f);
+  f.n = n;
+  f.per_layer = per;
+  f.ini_layers = ini;
+  f.kind = c->kind;
+  f.nparams = P.nparams;
+  f.nsweeps = layers * per;
+  f.cost = mc ? COST_NONE : c->cost_kind;
+  f.cost_maxabs = c->cost_maxabs;
+  f.cost_w0 = c->cost_w0;
+  for (int s = 0; s < per; ++s) {
+    f.t[s] = lay[s].t;
+    f.nact[s] = lay[s].k;
+    f.lo[s] = lay[s].lo;
+    f.off[s] = f.layer_bytes;
+    f.layer_bytes += fix_table_entries(lay[s].t, lay[s].k) * 16;
+  }
+  f.ctab_bytes = f.cost == COST_INT ? (2 * (int64_t)f.cost_maxabs + 1) * 16 : 0;
+  auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
+  f.tab0 = 0;
+  f.ctab0 = up(f.layer_bytes * layers);
+  f.startp = f.ctab0 + up(f.ctab_bytes * layers);
+  f.flags = f.startp + up((n + 1) * (int64_t)sizeof(double));
+  P.area_bytes = (size_t)(f.flags + up((int64_t)layers * per * (int64_t)sizeof(int32_t)));
+  const int8_t e = mc ? ent_of(c) : (int8_t)ENT_NONE;
+  P.periodic = mc && c->entangler == QG_ENT_CNOT_LADDER_PERIODIC;
+  P.first_param = ini * per;
+  P.fix.clear();
+  for (int i = 0; i < layers; ++i) {
+    const int li = i - ini;  // the circuit's layer (-1: the Ry(pi/4) layer)
+    for (int s = 0; s < per; ++s) {
+      P.fix.emplace_back();
+      FixDesc& d = P.fix.back();
+      memset(&d, 0, sizeof d);
+      d.n = n;
+      d.t = lay[s].t;
+      d.nact = lay[s].k;
+      d.nst = fix_stages(lay[s].k);
+      const int low = d.t - lay[s].k;
+      d.low = low;
+      d.lo = lay[s].lo;
+      const LadderMasks lm = ladder_masks(n, P.periodic);
+      d.odd = lm.odd;
+      d.even = lm.even;
+      for (int b = 0; b < FIX_E; ++b) {
+        const int j = d.t - FIX_E + b;  // local bit
+        d.top[b] = (int64_t)1 << (j < low ? j : lay[s].lo + j - low);
+        d.top_fwd[b] = (int64_t)ladder_fwd((uint64_t)d.top[b], lm);
+        d.top_inv[b] = (int64_t)ladder_inv((uint64_t)d.top[b], lm);
+      }
+      for (int a = 0; a < FIX_TMAX; ++a) d.slot[a] = -1;
+      for (int a = 0; a < lay[s].k; ++a) {
+        const int j = low + a, q = n - 1 - (lay[s].lo + a);
+        const int axis = li < 0 ? AX_Y : mc ? c->axes[(size_t)li * n + q] : AX_X;
+        if (li >= 0) d.slot[a] = mc ? li * n + q : li * (n + 1) + q;
+        // the stage and in-thread bit that hold local bit j
+        const int st = (d.t - 1 - j) / FIX_E, lo = d.t - FIX_E * (st + 1);
+        const int cb = lo >= 0 ? j - lo : j;
+        d.code[st] |= (uint8_t)((axis == AX_X ? 1 : axis == AX_Y ? 2 : 0) << (2 * cb));
+      }
+      d.gslot = -1;
+      d.start = START_LOAD;
+      d.periodic = P.periodic;
+      d.sweep = i * per + s;
+      d.tab = f.tab0 + i * f.layer_bytes + f.off[s];
+      d.ctab = f.ctab0 + i * f.ctab_bytes;
+      d.cost = COST_NONE;
+      d.cost_w0 = c->cost_w0;
+      d.cost_maxabs = c->cost_maxabs;
+      if (s == 0) {
+        d.pre = mc && (c->placement == QG_PLACE_BEFORE ? li >= 0 : li > 0) ? e : (int8_t)ENT_NONE;
+        if (!mc) d.cost = (int8_t)c->cost_kind;
+      }
+      if (!mc && s == per - 1 && li + 1 < c->L) {
+        // gamma of the next layer, at the end of this one (qaoa.py:65-68)
+        d.has_gslot = 1;
+        d.gslot = (li + 1) * (n + 1) + n;
+      }
+      fix_schedule(d);
+    }
+  }
+  if (!with_ini) P.fix[0].start = mc ? START_MCCLEAN : START_PLUS;
+  if (mc && c->placement == QG_PLACE_AFTER && c->L > 0) P.obs_pre = e;
+  P.fixed = true;
+}
+
+int build_program(const qg_circuit* c, int dtype, int op, bool with_ini, bool fixed, Program& P) {
   const int n = c->n;
   P.lay = make_layout(n, dtype, c->tune_tile_bits[dtype == QG_C64 ? 1 : 0]);
   P.sweeps.clear();
+  P.nparams = c->kind == 0 ? c->L * n : 2 * c->L;
+  P.nslots = c->kind == 0 ? P.nparams : c->L * (n + 1);
+  P.grad_kind = c->kind;
+  if (fixed) {
+    build_fixed(c, op, with_ini, P);
+    return QG_OK;
+  }
   if (c->kind == 0) {
-    P.nparams = c->L * n;
-    P.nslots = P.nparams;
-    P.grad_kind = 0;
     if (with_ini) {
       // Ry(pi/4) on every qubit of the caller's state (mc_clean.py:55-56)
       std::vector<LayerGate> g(n);
@@ -298,9 +486,7 @@ int build_program(const qg_circuit* c, int dtype, bool with_ini, Program& P) {
       if (st) return st;
     }
     P.first_param = (int)P.sweeps.size();
-    const int8_t e = (c->entangler == QG_ENT_CNOT_LADDER || c->entangler == QG_ENT_CNOT_LADDER_PERIODIC) ? ENT_CNOT
-                     : c->entangler == QG_ENT_CZ_LADDER                                          ? ENT_CZ
-                                                                                                 : ENT_NONE;
+    const int8_t e = ent_of(c);
     for (int i = 0; i < c->L; ++i) {
       std::vector<LayerGate> g(n);
       for (int q = 0; q < n; ++q) g[q] = LayerGate{c->axes[i * n + q], angle_param(i * n + q), i * n + q};
@@ -313,9 +499,6 @@ int build_program(const qg_circuit* c, int dtype, bool with_ini, Program& P) {
     if (c->placement == QG_PLACE_AFTER && c->L > 0) P.obs_pre = e;
   } else {
     const int p = c->L;
-    P.nparams = 2 * p;
-    P.nslots = p * (n + 1);
-    P.grad_kind = 1;
     P.first_param = 0;
     for (int i = 0; i < p; ++i) {
       std::vector<LayerGate> g(n);
@@ -401,7 +584,7 @@ struct ProfScope {
 };
 
 struct WsLayout {
-  size_t partials = 0, lam = 0, psi = 0, cost = 0, total = 0;
+  size_t partials = 0, lam = 0, psi = 0, cost = 0, area = 0, total = 0;
   size_t state_bytes = 0;
   int nstates_psi = 0;
   int nstates_lam = 0;
@@ -438,17 +621,29 @@ WsLayout ws_layout(const qg_circuit* c, int dtype, int op, const Program& P) {
   w.state_bytes = ((size_t)1 << n) * esz;
   const int64_t ntiles = (int64_t)1 << (n - P.lay.t);
   const int sms = sm_count();
+  const bool unc = op == QG_OP_GRAD_UNCOMPUTE;
+  const int tuned = c->tune_ctas[dtype == QG_C64 ? 1 : 0];
+  w.fwd_pipe = fwd_pipelined(c, dtype);
+  if (P.fixed) {
+    for (const auto& d : P.fix) {
+      const int64_t nt = (int64_t)1 << (n - d.t);
+      int pf = fix_ctas_per_sm(d.t, false, unc), pb = fix_ctas_per_sm(d.t, true, unc);
+      if (tuned > 0) pf = std::min(pf, tuned), pb = std::min(pb, tuned);
+      w.grid_fwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pf));
+      w.grid_bwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pb));
+      w.G = std::max(w.G, w.grid_bwd_k.back());
+    }
+    // the observable passes launch G CTAs of their own tiles
+    w.G = (int)std::max<int64_t>(w.G, std::min<int64_t>(ntiles, (int64_t)sms * 2));
+  } else {
   // resident CTAs per SM of the largest (shared-memory-wise) sweep
   SweepDesc big = P.sweeps[0];
   for (const auto& d : P.sweeps)
     if (d.nz > big.nz || (d.cost == COST_INT && big.cost != COST_INT)) big = d;
-  const bool unc = op == QG_OP_GRAD_UNCOMPUTE;
   int per_bwd = dtype == QG_C128 ? sweep_ctas_per_sm<double>(big, true, unc) : sweep_ctas_per_sm<float>(big, true, unc);
-  const bool pipe = fwd_pipelined(c, dtype);
-  w.fwd_pipe = pipe;
+  const bool pipe = w.fwd_pipe;
   int per_fwd = dtype == QG_C128 ? sweep_ctas_per_sm<double>(big, false, false, pipe)
                                  : sweep_ctas_per_sm<float>(big, false, false, pipe);
-  const int tuned = c->tune_ctas[dtype == QG_C64 ? 1 : 0];
   if (tuned > 0) {
     // never above what fits: the kernels assume every CTA of the grid is resident
     per_bwd = std::min(per_bwd, tuned);
@@ -488,10 +683,11 @@ WsLayout ws_layout(const qg_circuit* c, int dtype, int op, const Program& P) {
     }
     for (int g : w.grid_bwd_k) w.G = std::max(w.G, g);
   }
+  }
   w.neslots = obs_sweeps_needed(c, P.lay, op != QG_OP_RUN);
-  const int m = (int)P.sweeps.size();
+  const int m = P.nsweeps();
   w.pingpong = P.obs_pre == ENT_CNOT;
-  for (const auto& d : P.sweeps) w.pingpong = w.pingpong || d.pre == ENT_CNOT;
+  for (int k = 0; k < m; ++k) w.pingpong = w.pingpong || P.pre(k) == ENT_CNOT;
   const int two = w.pingpong ? 2 : 1;
   if (op == QG_OP_GRAD_HISTORY)
     w.nstates_psi = m;
@@ -512,6 +708,8 @@ WsLayout ws_layout(const qg_circuit* c, int dtype, int op, const Program& P) {
     else if (c->cost_kind == COST_REAL)
       off += align_up(((size_t)1 << n) * sizeof(double));
   }
+  w.area = off;
+  off += align_up(P.area_bytes);
   w.total = off;
   return w;
 }
@@ -530,14 +728,17 @@ struct Plan {
   std::vector<ObsDesc> obs;  // observable launches (lam stored for gradient ops)
 };
 
-// The cached plan of (current device, dtype, op, with_ini); built on first use.
-int get_plan(const qg_circuit* c, int dtype, int op, bool with_ini, std::shared_ptr<const Plan>& out) {
+// The cached plan of (current device, dtype, op, with_ini); built on first
+// use.  general: the double sweeps also where the fixed-point ones apply.
+int get_plan(const qg_circuit* c, int dtype, int op, bool with_ini, std::shared_ptr<const Plan>& out,
+             bool general = false) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
     dev = 0;
   }
-  const int key = ((dev * 2 + dtype) * 4 + op) * 2 + (with_ini ? 1 : 0);
+  const bool fixed = !general && fixed_path(c, dtype);
+  const int key = (((dev * 2 + dtype) * 4 + op) * 2 + (with_ini ? 1 : 0)) * 2 + (fixed ? 1 : 0);
   {
     std::lock_guard<std::mutex> lock(c->plan_mu);
     for (const auto& kv : c->plans)
@@ -547,12 +748,23 @@ int get_plan(const qg_circuit* c, int dtype, int op, bool with_ini, std::shared_
       }
   }
   auto plan = std::make_shared<Plan>();
-  if (int s = build_program(c, dtype, with_ini, plan->P)) return s;
+  if (int s = build_program(c, dtype, op, with_ini, fixed, plan->P)) return s;
   plan->W = ws_layout(c, dtype, op, plan->P);
   plan->obs = build_obs(c, plan->P, op != QG_OP_RUN, op != QG_OP_RUN, nullptr);
   std::lock_guard<std::mutex> lock(c->plan_mu);
   c->plans.emplace_back(key, plan);
   out = plan;
+  return QG_OK;
+}
+
+// The plan for a call with wsb bytes of workspace.  The fixed-point sweeps
+// keep their phase tables in it: a workspace that holds the double sweeps'
+// layout but not those (a fixed scratch size) runs the double sweeps.
+int plan_for(const qg_circuit* c, int dtype, int op, bool with_ini, size_t wsb, std::shared_ptr<const Plan>& out) {
+  if (int s = get_plan(c, dtype, op, with_ini, out)) return s;
+  if (wsb < out->W.total && out->P.fixed)
+    if (int s = get_plan(c, dtype, op, with_ini, out, true)) return s;
+  if (wsb < out->W.total) return fail(QG_ERR_WORKSPACE, "workspace %zu bytes < %zu needed", wsb, out->W.total);
   return QG_OK;
 }
 
@@ -666,6 +878,18 @@ int run_observable(const std::vector<ObsDesc>& obs, const WsLayout& W, const typ
   return QG_OK;
 }
 
+FixPtrs fix_ptrs(const Program& P, const WsLayout& W, char* ws) {
+  FixPtrs p;
+  memset(&p, 0, sizeof p);
+  p.area = ws + W.area;
+  p.cost_i = (const int32_t*)(ws + W.cost);
+  p.partials = (double*)(ws + W.partials);
+  p.flags = (const int32_t*)(ws + W.area + P.ft.flags);
+  p.startp = (const double*)(ws + W.area + P.ft.startp);
+  p.G = W.G;
+  return p;
+}
+
 template <typename R>
 int forward(const qg_circuit* c, const Program& P, const WsLayout& W, const double* params, const void* ini,
             bool history, char* ws, cudaStream_t st, const typename C2T<R>::T** final_state) {
@@ -680,21 +904,32 @@ int forward(const qg_circuit* c, const Program& P, const WsLayout& W, const doub
   const size_t N = (size_t)1 << c->n;
   C* buf[2] = {(C*)(ws + W.psi), W.pingpong && !history ? (C*)(ws + W.psi) + N : nullptr};
   int cur = 0;
-  const int m = (int)P.sweeps.size();
+  const int m = P.nsweeps();
   const C* in = (const C*)ini;
+  if (P.fixed) QG_CUDA(launch_fix_tables(P.ft, params, ws + W.area, st));
   for (int k = 0; k < m; ++k) {
     C* out;
     if (history) {
       out = buf[0] + (size_t)k * N;
     } else {
       // in place, except that a ladder gather reads other tiles: write the other buffer
-      if (P.sweeps[k].pre == ENT_CNOT && in == buf[cur]) cur ^= 1;
+      if (P.pre(k) == ENT_CNOT && in == buf[cur]) cur ^= 1;
       out = buf[cur];
     }
     p.psi_in = in;
     p.psi_out = out;
     ProfScope ps(0, st);
     // every sweep but the first follows a sweep launch: programmatic dependent
+    if constexpr (sizeof(R) == 8) {
+      if (P.fixed) {
+        FixPtrs q = fix_ptrs(P, W, ws);
+        q.psi_in = in;
+        q.psi_out = out;
+        QG_CUDA(launch_fix_fwd(P.fix[k], q, W.grid_fwd_k[k], st, k > 0));
+        in = out;
+        continue;
+      }
+    }
     QG_CUDA(launch_sweep_fwd<R>(P.sweeps[k], p, W.grid_fwd_k[k], st, W.fwd_pipe, k > 0));
     in = out;
   }
@@ -707,17 +942,16 @@ int do_run(const qg_circuit* c, const double* params, const void* ini, char* ws,
            void* state_out, cudaStream_t st, int dtype) {
   using C = typename C2T<R>::T;
   std::shared_ptr<const Plan> plan;
-  int s = get_plan(c, dtype, QG_OP_RUN, ini != nullptr, plan);
+  int s = plan_for(c, dtype, QG_OP_RUN, ini != nullptr, wsb, plan);
   if (s) return s;
   const Program& P = plan->P;
   const WsLayout& W = plan->W;
-  if (wsb < W.total) return fail(QG_ERR_WORKSPACE, "workspace %zu bytes < %zu needed", wsb, W.total);
   s = build_cost(c, ws, W, st);
   if (s) return s;
   const C* fin = nullptr;
   s = forward<R>(c, P, W, params, ini, false, ws, st, &fin);
   if (s) return s;
-  s = run_observable<R>(plan->obs, W, fin, nullptr, ws, st, !P.sweeps.empty());
+  s = run_observable<R>(plan->obs, W, fin, nullptr, ws, st, P.nsweeps() > 0);
   if (s) return s;
   QG_CUDA(launch_finalize((double*)(ws + W.partials), W.G, 0, c->n, 0, P.nslots, W.neslots, expec, nullptr, st));
   if (state_out) QG_CUDA(cudaMemcpyAsync(state_out, fin, W.state_bytes, cudaMemcpyDeviceToDevice, st));
@@ -731,11 +965,10 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
             double* grad, cudaStream_t st, int dtype, int component = -1) {
   using C = typename C2T<R>::T;
   std::shared_ptr<const Plan> plan;
-  int s = get_plan(c, dtype, op, ini != nullptr, plan);
+  int s = plan_for(c, dtype, op, ini != nullptr, wsb, plan);
   if (s) return s;
   const Program& P = plan->P;
   const WsLayout& W = plan->W;
-  if (wsb < W.total) return fail(QG_ERR_WORKSPACE, "workspace %zu bytes < %zu needed", wsb, W.total);
   const bool history = op == QG_OP_GRAD_HISTORY;
   QG_CUDA(cudaMemsetAsync(ws + W.partials, 0, (size_t)(P.nslots + W.neslots) * W.G * sizeof(double), st));
   s = build_cost(c, ws, W, st);
@@ -753,11 +986,11 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
     // overwritten by the full-observable pass, which writes at least the
     // same slots, so E stays <psi|O|psi> (mc_clean.py:99-100)
     const std::vector<Term> one(1, c->terms[component]);
-    s = run_observable<R>(build_obs(c, P, true, true, &one), W, fin, lbuf[lc], ws, st, !P.sweeps.empty());
+    s = run_observable<R>(build_obs(c, P, true, true, &one), W, fin, lbuf[lc], ws, st, P.nsweeps() > 0);
     if (s) return s;
     s = run_observable<R>(build_obs(c, P, false, false, nullptr), W, fin, nullptr, ws, st, true);
   } else {
-    s = run_observable<R>(plan->obs, W, fin, lbuf[lc], ws, st, !P.sweeps.empty());
+    s = run_observable<R>(plan->obs, W, fin, lbuf[lc], ws, st, P.nsweeps() > 0);
   }
   if (s) return s;
   SweepPtrs<R> p;
@@ -768,24 +1001,40 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
   p.partials = (double*)(ws + W.partials);
   p.G = W.G;
   C* psi0 = (C*)(ws + W.psi);
-  const int m = (int)P.sweeps.size();
+  const int m = P.nsweeps();
   for (int k = m - 1; k >= P.first_param; --k) {
-    SweepDesc d = P.sweeps[k];
     // undo, on load, the entangler the forward applied right after sweep k
-    d.lam_undo = k + 1 < m ? P.sweeps[k + 1].pre : P.obs_pre;
-    d.psi_undo = history ? ENT_NONE : (k + 1 < m ? P.sweeps[k + 1].pre : ENT_NONE);
+    const int8_t lam_undo = k + 1 < m ? P.pre(k + 1) : P.obs_pre;
+    const int8_t psi_undo = history ? (int8_t)ENT_NONE : (k + 1 < m ? P.pre(k + 1) : (int8_t)ENT_NONE);
     p.lam_in = lbuf[lc];
-    if (d.lam_undo == ENT_CNOT) lc ^= 1;
+    if (lam_undo == ENT_CNOT) lc ^= 1;
     p.lam_out = lbuf[lc];
     if (history) {
       p.psi_in = psi0 + (size_t)k * N;
       p.psi_out = nullptr;
     } else {
       p.psi_in = pbuf[pc];
-      if (d.psi_undo == ENT_CNOT) pc ^= 1;
+      if (psi_undo == ENT_CNOT) pc ^= 1;
       p.psi_out = pbuf[pc];
     }
     ProfScope ps(1, st);
+    if constexpr (sizeof(R) == 8) {
+      if (P.fixed) {
+        FixDesc d = P.fix[k];
+        d.lam_undo = lam_undo;
+        d.psi_undo = psi_undo;
+        FixPtrs q = fix_ptrs(P, W, ws);
+        q.psi_in = p.psi_in;
+        q.psi_out = p.psi_out;
+        q.lam_in = p.lam_in;
+        q.lam_out = p.lam_out;
+        QG_CUDA(launch_fix_bwd(d, q, !history, W.grid_bwd_k[k], st, true));
+        continue;
+      }
+    }
+    SweepDesc d = P.sweeps[k];
+    d.lam_undo = lam_undo;
+    d.psi_undo = psi_undo;
     // follows the observable pass or the previous backward sweep
     QG_CUDA(launch_sweep_bwd<R>(d, p, !history, W.grid_bwd_k[k], st, true));
   }
@@ -821,6 +1070,14 @@ int parse_terms(int n, int nterms, const int32_t* kind, const int32_t* q0, const
 
 namespace qg {
 int set_last_error(int status, const char* msg) { return fail(status, "%s", msg); }
+
+int min_workspace(const qg_circuit* c, int dtype, int op, size_t* bytes) {
+  if (int s = qg_workspace_size(c, dtype, op, bytes)) return s;
+  std::shared_ptr<const Plan> plan;
+  if (int s = get_plan(c, dtype, op, c->kind == 0, plan, true)) return s;
+  *bytes = std::min(*bytes, plan->W.total);
+  return QG_OK;
+}
 }  // namespace qg
 
 extern "C" {

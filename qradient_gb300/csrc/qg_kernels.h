@@ -2,12 +2,15 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "../../include/qgrad.h"
 #include "qg_internal.cuh"
 
 namespace qg {
 
 // Record a failure message for qg_last_error() and return the status.
 int set_last_error(int status, const char* msg);
+// the smallest workspace qg_run / qg_grad accept for an op (qg_capi.cu)
+int min_workspace(const qg_circuit* c, int dtype, int op, size_t* bytes);
 
 // Resident CTAs per SM of a sweep kernel with this descriptor's shared memory
 // (pipe: the double-buffered forward kernel).

@@ -73,7 +73,8 @@ int scratch_address(void** out) {
 extern "C" int qg_grad_noalloc(const qg_circuit* c, int dtype, const double* params_dev, const void* ini_state_dev,
                                double* expec_dev, double* grad_dev, qg_stream stream) {
   size_t need = 0;
-  int st = qg_workspace_size(c, dtype, QG_OP_GRAD_UNCOMPUTE, &need);
+  // (the smallest layout qg_grad accepts: without the fixed-point sweeps' tables)
+  int st = qg::min_workspace(c, dtype, QG_OP_GRAD_UNCOMPUTE, &need);
   if (st != QG_OK) return st;
   if (need > kScratchBytes) {
     char msg[256];
