@@ -200,12 +200,20 @@ class Batch:
         idx = np.asarray(cols["i"], dtype=np.int64)
         qn = np.asarray(cols["n"], dtype=np.int64)
         per = np.asarray(cols["periodic"], dtype=bool)
+        # launch groups, the smallest jobs first.  A complex128 launch runs every
+        # job in a block of the launch's size (2^9 amplitudes at least), so its
+        # jobs are grouped by size as well; complex64 jobs of a cluster size
+        # share one launch
         groups = []
         pair = PAIR_MAX[self.dtype]
-        for cl, sel in ((1, (qn < split) | per), (2, (qn >= split) & (qn <= pair) & ~per), (4, (qn > pair) & ~per)):
-            nj = int(sel.sum()) if idx.size else 0
-            if nj:
-                groups.append((cl, sel, nj, int(qn[sel].max())))
+        for cl, lg, sel in ((1, 0, (qn < split) | per), (2, 1, (qn >= split) & (qn <= pair) & ~per),
+                            (4, 2, (qn > pair) & ~per)):
+            if not idx.size or not sel.any():
+                continue
+            block = np.maximum(qn - lg, 9) if self.dtype == _lib.QG_C128 else np.zeros_like(qn)
+            for b in np.unique(block[sel]):
+                part = sel & (block == b)
+                groups.append((cl, part, int(part.sum()), int(qn[part].max())))
         # layout of the upload: params | structures | job tables | job counters
         size = 0
         p_off = None
@@ -288,10 +296,32 @@ class Batch:
     # ------------------------------------------------------------ execution
     def _launch(self):
         lib = _lib.load()
-        stream = _native.stream_handle(self.device)
-        for cl, jobs, nj, maxq, ws in self._groups:
+
+        def launch(group):
+            cl, jobs, nj, maxq, ws = group
             _lib.check(lib.qg_batch_launch(self.dtype, _native.ptr(jobs), nj, maxq, cl, _native.ptr(ws), ws.numel(),
-                                           stream))
+                                           _native.stream_handle(self.device)))
+
+        # The groups are independent: all but one go to streams of their own,
+        # forked from and joined to the current one, so that a small batch
+        # takes as long as its longest job, not the sum over its groups (96
+        # complex128 jobs of 8..14 qubits: 6.9 -> 3.9 ms).  Longest jobs first.
+        main = torch.cuda.current_stream(self.device)
+        groups = self._groups[::-1]
+        side = []
+        if len(groups) > 1:
+            fork = torch.cuda.Event()
+            fork.record(main)
+            for group in groups[1:]:
+                st = torch.cuda.Stream(self.device)
+                st.wait_event(fork)
+                side.append((st, group))
+        for group in groups[:1]:
+            launch(group)
+        for st, group in side:
+            with torch.cuda.stream(st):
+                launch(group)
+            main.wait_stream(st)
         for i in self._big:
             s = self._specs[i]
             c = s["circuit"]

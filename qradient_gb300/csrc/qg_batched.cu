@@ -1,22 +1,22 @@
-// Batched persistent kernel: many small circuits (different parameters,
-// qubit counts, depths, McClean or QAOA) in one launch.
+// Batched persistent kernel in complex64: many small circuits (different
+// parameters, qubit counts, depths, McClean or QAOA) in one launch.  (The
+// complex128 form is qg_batched_fix.cu.)
 //
 // Each job is a whole run or adjoint grad_run (mc_clean.py:27-78,
 // qaoa.py:23-70) executed with psi and lambda resident in shared memory:
 // no state ever goes to HBM.  A CTA holds the whole state when it fits
-// (complex64 n <= 13, complex128 n <= 12); a 2-CTA cluster holds one state
-// split by its top bit (qubit 0) at the next size (complex64 n = 14,
-// complex128 n = 13) and a 4-CTA cluster, split by its top two bits, at the
-// one after (complex64 n = 15, complex128 n = 14).  The only cross-CTA
-// operations (rotations, reductions and X/Y observable terms on the split
-// qubits) read the partner CTA's shared memory (distributed shared memory)
-// between cluster barriers.  The CNOT ladder never targets qubit 0; its
-// CNOT(0, 1) permutes the 4-CTA blocks, which the CTAs follow by relabelling.
+// (n <= 13); a 2-CTA cluster holds one state split by its top bit (qubit 0)
+// at the next size (n = 14) and a 4-CTA cluster, split by its top two bits,
+// at the one after (n = 15).  The only cross-CTA operations (rotations,
+// reductions and X/Y observable terms on the split qubits) read the partner
+// CTA's shared memory (distributed shared memory) between cluster barriers.
+// The CNOT ladder never targets qubit 0; its CNOT(0, 1) permutes the 4-CTA
+// blocks, which the CTAs follow by relabelling.
 //
 // Clusters (or CTAs) take jobs from a device counter until the queue is
-// empty (persistent grid, one launch per precision and cluster size; the
-// launch is CUDA-graph capturable).  The gradient uses the uncompute form of
-// the adjoint sweep (psi is rotated back instead of read from a history).
+// empty (persistent grid, one launch per cluster size; the launch is
+// CUDA-graph capturable).  The gradient uses the uncompute form of the
+// adjoint sweep (psi is rotated back instead of read from a history).
 #include <cooperative_groups.h>
 #include <stdint.h>
 
@@ -32,21 +32,16 @@ constexpr int BZMAX = 10;     // Z rotations merged per table (2^BZMAX = BATCH_T
 constexpr int BMAXQ = 26;
 constexpr int BTERMS = 64;    // observable weights staged in shared memory
 
-__device__ __forceinline__ double2 cmulb(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
 __device__ __forceinline__ float2 cmulb(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 __device__ __forceinline__ float2 tocf(float x, float y) { return make_float2(x, y); }
-__device__ __forceinline__ double2 tocf(double x, double y) { return make_double2(x, y); }
-__device__ __forceinline__ void sincosT(double a, double* s, double* c) { sincos(a, s, c); }
 __device__ __forceinline__ void sincosT(float a, float* s, float* c) { sincosf(a, s, c); }
 
-// XOR swizzle of the low index bits with the next ones: 8 (complex128) or 16
-// (complex64) amplitudes per 128-byte row, so tasks that stride over the low
-// bits still spread over all banks
-__device__ __forceinline__ int swb(int e, bool dbl) { return dbl ? e ^ ((e >> 3) & 7) : e ^ ((e >> 4) & 15); }
+// XOR swizzle of the low index bits with the next ones: 16 amplitudes per
+// 128-byte row, so tasks that stride over the low bits still spread over all
+// banks
+__device__ __forceinline__ int swb(int e) { return e ^ ((e >> 4) & 15); }
 __device__ __forceinline__ int ins0(int p, int j) { return ((p >> j) << (j + 1)) | (p & ((1 << j) - 1)); }
 
 // index arithmetic of the batched kernel is 32-bit: its jobs have at most 26
@@ -65,8 +60,8 @@ __device__ __forceinline__ uint32_t lad_inv(uint32_t x, uint32_t odd, uint32_t e
 }
 
 // Scaled form of a rotation by theta, in the precision T of the job's
-// coefficients (double for complex128, float for complex64: a double
-// instruction holds the FP64 pipe for 16 cycles per warp).
+// coefficients (float: a double instruction holds the FP64 pipe for 16 cycles
+// per warp).
 template <typename T>
 __device__ __forceinline__ T rform(T theta, int* form, T* kappa) {
   T s, c;
@@ -161,8 +156,8 @@ __device__ __forceinline__ R wsum(R v) {
 
 // G rotations on ascending local bits bits[0..G-1], each thread owning the
 // 2^G amplitudes of one task (all other bits fixed) in registers.
-template <typename C, typename R, int G, int NT, bool DBL, int SG>
-__device__ __forceinline__ void rot_group(C* v, C* v2, int M, const int* bits, const int* axis, const int* form,
+template <typename C, typename R, int G, int NT, int SG>
+__device__ __forceinline__ void rot_group(C* v, int M, const int* bits, const int* axis, const int* form,
                                           const R* u) {
   const int ntask = M >> G;
   int b[G];
@@ -179,12 +174,12 @@ __device__ __forceinline__ void rot_group(C* v, C* v2, int M, const int* bits, c
   // XOR the swizzled group bits
   int sbit[G];
 #pragma unroll
-  for (int i = 0; i < G; ++i) sbit[i] = swb(1 << b[i], DBL);
+  for (int i = 0; i < G; ++i) sbit[i] = swb(1 << b[i]);
   for (int tk = threadIdx.x; tk < ntask; tk += NT) {
     int base = tk;
 #pragma unroll
     for (int i = 0; i < G; ++i) base = ins0(base, b[i]);
-    const int sb = swb(base, DBL);
+    const int sb = swb(base);
     int idx[1 << G];
 #pragma unroll
     for (int c = 0; c < (1 << G); ++c) {
@@ -194,73 +189,14 @@ __device__ __forceinline__ void rot_group(C* v, C* v2, int M, const int* bits, c
         if ((c >> i) & 1) x ^= sbit[i];
       idx[c] = x;
     }
+    C el[1 << G];
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      C* w = pass ? v2 : v;
-      if (w == nullptr) break;
-      C el[1 << G];
+    for (int c = 0; c < (1 << G); ++c) el[c] = v[idx[c]];
+    rotb_any<SG, 0, G>(el, ax[0], fm[0], uu[0]);
+    if (G > 1) rotb_any<SG, (G > 1 ? 1 : 0), G>(el, ax[G > 1 ? 1 : 0], fm[G > 1 ? 1 : 0], uu[G > 1 ? 1 : 0]);
+    if (G > 2) rotb_any<SG, (G > 2 ? 2 : 0), G>(el, ax[G > 2 ? 2 : 0], fm[G > 2 ? 2 : 0], uu[G > 2 ? 2 : 0]);
 #pragma unroll
-      for (int c = 0; c < (1 << G); ++c) el[c] = w[idx[c]];
-      rotb_any<SG, 0, G>(el, ax[0], fm[0], uu[0]);
-      if (G > 1) rotb_any<SG, (G > 1 ? 1 : 0), G>(el, ax[G > 1 ? 1 : 0], fm[G > 1 ? 1 : 0], uu[G > 1 ? 1 : 0]);
-      if (G > 2) rotb_any<SG, (G > 2 ? 2 : 0), G>(el, ax[G > 2 ? 2 : 0], fm[G > 2 ? 2 : 0], uu[G > 2 ? 2 : 0]);
-#pragma unroll
-      for (int c = 0; c < (1 << G); ++c) w[idx[c]] = el[c];
-    }
-  }
-}
-
-// Gradient reductions of G rotations on ascending bits from one pass over
-// the 2^G-amplitude tasks (lambda and psi in registers); the warp sums land
-// in out[0..G-1] (this warp's reduction slots).
-template <typename C, typename R, int G, int NT, bool DBL>
-__device__ __forceinline__ void red_group(const C* lam, const C* psi, int M, const int* bits, const int* axis,
-                                          R* out) {
-  int b[G], ax[G];
-  R acc[G];
-#pragma unroll
-  for (int i = 0; i < G; ++i) {
-    b[i] = bits[i];
-    ax[i] = axis[i];
-    acc[i] = (R)0;
-  }
-  const int ntask = M >> G;
-  int sbit[G];
-#pragma unroll
-  for (int i = 0; i < G; ++i) sbit[i] = swb(1 << b[i], DBL);
-  for (int tk = threadIdx.x; tk < ntask; tk += NT) {
-    int base = tk;
-#pragma unroll
-    for (int i = 0; i < G; ++i) base = ins0(base, b[i]);
-    const int sb = swb(base, DBL);
-    C la[1 << G], qa[1 << G];
-#pragma unroll
-    for (int c = 0; c < (1 << G); ++c) {
-      int x = sb;
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        if ((c >> i) & 1) x ^= sbit[i];
-      la[c] = lam[x];
-      qa[c] = psi[x];
-    }
-#pragma unroll
-    for (int i = 0; i < G; ++i) {
-      // warp-uniform branch around the whole unrolled block
-      if (ax[i] == 0) {
-#pragma unroll
-        for (int c = 0; c < (1 << G); ++c)
-          if (!((c >> i) & 1)) acc[i] += redp<C, R>(la[c], la[c | (1 << i)], qa[c], qa[c | (1 << i)], 0);
-      } else {
-#pragma unroll
-        for (int c = 0; c < (1 << G); ++c)
-          if (!((c >> i) & 1)) acc[i] += redp<C, R>(la[c], la[c | (1 << i)], qa[c], qa[c | (1 << i)], 1);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < G; ++i) {
-    const R v = wsum(acc[i]);
-    if ((threadIdx.x & 31) == 0) out[i] = v;
+    for (int c = 0; c < (1 << G); ++c) v[idx[c]] = el[c];
   }
 }
 
@@ -272,7 +208,7 @@ __device__ __forceinline__ void red_group(const C* lam, const C* psi, int M, con
 // The scaled forms divide each state by the rotation's kappa, so sums taken
 // after earlier groups carry 1 / prod(kappa^2) of those groups: `scale`
 // (that product) restores them.
-template <typename C, typename R, int G, int NT, bool DBL>
+template <typename C, typename R, int G, int NT>
 __device__ __forceinline__ void rotred_group(C* lam, C* psi, int M, const int* bits, const int* axis, const int* form,
                                              const R* u, R scale, R* out) {
   int b[G], ax[G], fm[G];
@@ -287,13 +223,13 @@ __device__ __forceinline__ void rotred_group(C* lam, C* psi, int M, const int* b
   }
   int sbit[G];
 #pragma unroll
-  for (int i = 0; i < G; ++i) sbit[i] = swb(1 << b[i], DBL);
+  for (int i = 0; i < G; ++i) sbit[i] = swb(1 << b[i]);
   const int ntask = M >> G;
   for (int tk = threadIdx.x; tk < ntask; tk += NT) {
     int base = tk;
 #pragma unroll
     for (int i = 0; i < G; ++i) base = ins0(base, b[i]);
-    const int sb = swb(base, DBL);
+    const int sb = swb(base);
     int idx[1 << G];
 #pragma unroll
     for (int c = 0; c < (1 << G); ++c) {
@@ -374,7 +310,6 @@ template <typename R, int CS, int NT>
 __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restrict__ jobs, int njobs, int* counter,
                                                       int mmax) {
   using C = typename BatchC<R>::T;
-  constexpr bool DBL = sizeof(R) == 8;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ BShared<R> S;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -488,7 +423,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       C v;
       v.x = J.kind == 0 ? (R)S.startP[__popc(x)] : plus;
       v.y = (R)0;
-      psi[swb(e, DBL)] = v;
+      psi[swb(e)] = v;
     }
     __syncthreads();
 
@@ -567,13 +502,12 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       }
       __syncthreads();
     };
-    // diagonal of layer i (Z table * K; QAOA cost phase * K); conj for the inverse.
-    // The Z table is built by doubling: 2^nz complex multiplies in all.
+    // diagonal of layer i (Z table * K; QAOA cost phase * K); conj for the inverse
     auto build_diag = [&](int i, bool inv) {
       const int nzt = S.nz < BZMAX ? S.nz : BZMAX;
-      if (J.kind == 0 && !DBL) {
-        // complex64: every entry as its own product (nzt float multiplies),
-        // one barrier instead of one per Z rotation
+      if (J.kind == 0) {
+        // every entry as its own product (nzt float multiplies), one barrier
+        // instead of one per Z rotation by doubling
         for (int pp = tid; pp < (1 << nzt); pp += NT) {
           C v = tocf(S.K, (R)0);
           for (int j = 0; j < nzt; ++j) {
@@ -583,21 +517,6 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
             v = cmulb(v, tocf(S.zc[j], sg * S.zs[j]));
           }
           ztab[pp] = v;
-        }
-      } else if (J.kind == 0) {
-        // complex128: doubling, 2^nzt complex multiplies in all
-        if (tid == 0) ztab[0] = tocf(S.K, (R)0);
-        __syncthreads();
-        for (int j = 0; j < nzt; ++j) {
-          const int h = 1 << j;
-          const C e0 = tocf(S.zc[j], inv ? S.zs[j] : -S.zs[j]);
-          const C e1 = tocf(S.zc[j], inv ? -S.zs[j] : S.zs[j]);
-          for (int pp = tid; pp < h; pp += NT) {
-            const C v = ztab[pp];
-            ztab[pp + h] = cmulb(v, e1);
-            ztab[pp] = cmulb(v, e0);
-          }
-          __syncthreads();
         }
       } else {
         const R g = (R)(J.params[2 * i + 1] * J.cost_w0);
@@ -642,7 +561,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         for (int j = 0; j < nzt; ++j) ptid |= (int)(((uint32_t)tid >> S.zbit[j]) & 1) << j;
       for (int e = tid, k = 0; e < M; e += NT, ++k) {
         const uint32_t x = top | (uint32_t)e;
-        C a = v[swb(e, DBL)];
+        C a = v[swb(e)];
         if (J.kind == 0) {
           a = cmulb(a, ztab[ptid | S.zpk[k]]);
           for (int j = BZMAX; j < S.nz; ++j) {
@@ -653,7 +572,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         } else {
           a = cmulb(a, ztab[cost_m(x) + J.cost_maxabs]);
         }
-        v[swb(e, DBL)] = a;
+        v[swb(e)] = a;
       }
       __syncthreads();
     };
@@ -664,10 +583,10 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         for (int e = tid; e < M; e += NT) {
           const uint32_t x = top | (uint32_t)e;
           if (__popc(x & (x >> 1)) & 1) {
-            C a = v[swb(e, DBL)];
+            C a = v[swb(e)];
             a.x = -a.x;
             a.y = -a.y;
-            v[swb(e, DBL)] = a;
+            v[swb(e)] = a;
           }
         }
         __syncthreads();
@@ -676,7 +595,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       for (int e = tid; e < M; e += NT) {
         const uint32_t x = top | (uint32_t)e;
         const uint32_t src = inv ? lad_fwd(x, lodd, leven, lwrap, lws) : lad_inv(x, lodd, leven, lwrap, lws);
-        scr[swb(e, DBL)] = v[swb((int)(src & (uint32_t)(M - 1)), DBL)];
+        scr[swb(e)] = v[swb((int)(src & (uint32_t)(M - 1)))];
       }
       __syncthreads();
       C* t = v;
@@ -697,14 +616,14 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
           cluster.sync();
           const C* rw = rmt(w, lrank ^ (1 << cb));
           for (int e = tid; e < M; e += NT) {
-            const C own = w[swb(e, DBL)];
-            const C rem = rw[swb(e, DBL)];
+            const C own = w[swb(e)];
+            const C rem = rw[swb(e)];
             C x0 = low ? own : rem, x1 = low ? rem : own;
             if (inverse)
               rotp<-1, C, R>(x0, x1, S.caxis[c], S.cform[c], (R)S.cu[c]);
             else
               rotp<1, C, R>(x0, x1, S.caxis[c], S.cform[c], (R)S.cu[c]);
-            scr[swb(e, DBL)] = low ? x0 : x1;
+            scr[swb(e)] = low ? x0 : x1;
           }
           cluster.sync();
           C* t = w;
@@ -713,30 +632,20 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         }
       }
     };
-    auto rotate = [&](C*& v, C* v2in, bool inverse) {
-      C* v2 = v2in;
+    auto rotate = [&](C*& v) {
       const int nxy = S.nxy;
       for (int g0 = 0; g0 < nxy; g0 += 3) {
         const int g = nxy - g0 < 3 ? nxy - g0 : 3;
-        if (!inverse) {
-          if (g == 3)
-            rot_group<C, R, 3, NT, DBL, 1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-          else if (g == 2)
-            rot_group<C, R, 2, NT, DBL, 1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-          else
-            rot_group<C, R, 1, NT, DBL, 1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-        } else {
-          if (g == 3)
-            rot_group<C, R, 3, NT, DBL, -1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-          else if (g == 2)
-            rot_group<C, R, 2, NT, DBL, -1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-          else
-            rot_group<C, R, 1, NT, DBL, -1>(v, v2, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
-        }
+        if (g == 3)
+          rot_group<C, R, 3, NT, 1>(v, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
+        else if (g == 2)
+          rot_group<C, R, 2, NT, 1>(v, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
+        else
+          rot_group<C, R, 1, NT, 1>(v, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0);
         __syncthreads();
       }
-      rotate_cross(v, v2, inverse);
-      return v2;
+      C* none = nullptr;
+      rotate_cross(v, none, false);
     };
 
     // block-sum of one value into the job's output (with 2 CTAs: two atomic
@@ -772,12 +681,12 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         // CZ: a sign, its own inverse, in place
         for (int e = tid, k = 0; e < M; e += NT, ++k) {
           const uint32_t x = top | (uint32_t)e;
-          C a = cmulb(v[swb(e, DBL)], ztab[ptid | S.zpk[k]]);
+          C a = cmulb(v[swb(e)], ztab[ptid | S.zpk[k]]);
           if (__popc(x & (x >> 1)) & 1) {
             a.x = -a.x;
             a.y = -a.y;
           }
-          v[swb(e, DBL)] = a;
+          v[swb(e)] = a;
         }
         __syncthreads();
         return;
@@ -786,7 +695,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         const uint32_t x = top | (uint32_t)e;
         const uint32_t src = inv ? lad_fwd(x, lodd, leven, lwrap, lws) : lad_inv(x, lodd, leven, lwrap, lws);
         const int pat = inv ? (ptid ^ S.zpkf[k]) : (ptid | S.zpk[k]);
-        scr[swb(e, DBL)] = cmulb(v[swb((int)(src & (uint32_t)(M - 1)), DBL)], ztab[pat]);
+        scr[swb(e)] = cmulb(v[swb((int)(src & (uint32_t)(M - 1)))], ztab[pat]);
       }
       __syncthreads();
       C* t = v;
@@ -813,7 +722,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       }
       // (no cluster barrier here: the only cross-CTA reads of a layer,
       // rotate_cross's, sit between barriers of their own)
-      rotate(psi, nullptr, false);
+      rotate(psi);
       if (J.kind == 0 && J.entangler != 0 && J.placement == 1) {
         if (ladder) relabel();
         entangle(psi, false);
@@ -827,7 +736,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       const bool costonly = J.kind == 1 && grad;
       for (int e = tid; e < M; e += NT) {
         const uint32_t x = top | (uint32_t)e;
-        const C v = psi[swb(e, DBL)];
+        const C v = psi[swb(e)];
         R lx = (R)0, ly = (R)0;
         if (costonly) {
           const R d = (R)J.cost_w0 * (R)cost_m(x);
@@ -848,9 +757,9 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
               const uint32_t xp = x ^ b0;
               C u;
               if ((xp >> m) != (x >> m))
-                u = rmt(psi, (int)(xp >> m))[swb((int)(xp & (uint32_t)(M - 1)), DBL)];
+                u = rmt(psi, (int)(xp >> m))[swb((int)(xp & (uint32_t)(M - 1)))];
               else
-                u = psi[swb((int)(xp & (uint32_t)(M - 1)), DBL)];
+                u = psi[swb((int)(xp & (uint32_t)(M - 1)))];
               const R w = tw;
               if (t.kind == 0) {
                 lx = fma(w, u.x, lx);
@@ -868,7 +777,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
           C o;
           o.x = lx;
           o.y = ly;
-          lam[swb(e, DBL)] = o;
+          lam[swb(e)] = o;
         }
       }
       const R v = wsum(eacc);
@@ -894,7 +803,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         R acc = (R)0;
         for (int e = tid; e < M; e += NT) {
           const uint32_t x = top | (uint32_t)e;
-          const C v = psi[swb(e, DBL)];
+          const C v = psi[swb(e)];
           if (t.kind >= 2) {
             bool sg = (x & b0) != 0;
             if (t.kind == 3) sg ^= (x & (1u << (n - 1 - t.q1))) != 0;
@@ -902,8 +811,8 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
             acc += sg ? -p2 : p2;
           } else {
             const uint32_t xp = x ^ b0;
-            const C u = (xp >> m) != (x >> m) ? rmt(psi, (int)(xp >> m))[swb((int)(xp & (uint32_t)(M - 1)), DBL)]
-                                              : psi[swb((int)(xp & (uint32_t)(M - 1)), DBL)];
+            const C u = (xp >> m) != (x >> m) ? rmt(psi, (int)(xp >> m))[swb((int)(xp & (uint32_t)(M - 1)))]
+                                              : psi[swb((int)(xp & (uint32_t)(M - 1)))];
             if (t.kind == 0) {
               acc += fma(v.x, u.x, v.y * u.y);  // Re(conj(v) u)
             } else {
@@ -944,29 +853,16 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
         // rotations and are taken afterwards.
         const int nxy = S.nxy;
         R sc = (R)1;  // prod kappa^2 of the rotations already applied
-        if (DBL) {
-          // complex128: separate reduction passes at the layer's end point;
-          // the fused form needs more than the 128 registers a thread has here
-          for (int g0 = 0; g0 < nxy; g0 += 3) {
-            const int g = nxy - g0 < 3 ? nxy - g0 : 3;
-            if (g == 3)
-              red_group<C, R, 3, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, &S.red[warp][g0]);
-            else if (g == 2)
-              red_group<C, R, 2, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, &S.red[warp][g0]);
-            else
-              red_group<C, R, 1, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, &S.red[warp][g0]);
-          }
-        }
-        for (int g0 = 0; !DBL && g0 < nxy; g0 += 3) {
+        for (int g0 = 0; g0 < nxy; g0 += 3) {
           const int g = nxy - g0 < 3 ? nxy - g0 : 3;
           if (g == 3)
-            rotred_group<C, R, 3, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
+            rotred_group<C, R, 3, NT>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
                                            &S.red[warp][g0]);
           else if (g == 2)
-            rotred_group<C, R, 2, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
+            rotred_group<C, R, 2, NT>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
                                            &S.red[warp][g0]);
           else
-            rotred_group<C, R, 1, NT, DBL>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
+            rotred_group<C, R, 1, NT>(lam, psi, M, S.xbit + g0, S.xaxis + g0, S.xform + g0, S.xu + g0, sc,
                                            &S.red[warp][g0]);
           for (int i = g0; i < g0 + g; ++i) sc *= S.xk[i] * S.xk[i];
           __syncthreads();
@@ -980,8 +876,8 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
           const C* rq = rmt(psi, lrank ^ (1 << cb));
           R a = (R)0;
           for (int e = tid; e < M; e += NT) {
-            const C l = lam[swb(e, DBL)];
-            const C qr = rq[swb(e, DBL)];
+            const C l = lam[swb(e)];
+            const C qr = rq[swb(e)];
             if (S.caxis[c] == 0)
               a += fma(l.x, qr.y, -l.y * qr.x);
             else
@@ -1000,7 +896,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
           R T = (R)0;
           R Uk[4] = {(R)0, (R)0, (R)0, (R)0};
           for (int e = tid, k = 0; e < M; e += NT, ++k) {
-            const C l = lam[swb(e, DBL)], q = psi[swb(e, DBL)];
+            const C l = lam[swb(e)], q = psi[swb(e)];
             const R w = fma(l.x, q.y, -l.y * q.x);
             T += w;
 #pragma unroll
@@ -1043,14 +939,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
             J.grad[2 * i] = (double)tot;
         }
         __syncthreads();
-        // complex128 rotates psi here before rotate_cross's first barrier:
-        // the partners may still read it for their cross reductions
-        if (CS > 1 && DBL && ncr) cluster.sync();
-        // inverse rotations on lam and psi
-        if (DBL)
-          psi = rotate(lam, psi, true);
-        else
-          rotate_cross(lam, psi, true);
+        rotate_cross(lam, psi, true);
         const bool fz = fuse && S.nz <= BZMAX;
         if (fz && ladder) relabel();  // the fused table reads the new block's index
         build_diag(i, true);
@@ -1067,7 +956,7 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
           R gsum = (R)0;
           for (int e = tid; e < M; e += NT) {
             const uint32_t x = top | (uint32_t)e;
-            const C l = lam[swb(e, DBL)], q = psi[swb(e, DBL)];
+            const C l = lam[swb(e)], q = psi[swb(e)];
             gsum = fma((R)J.cost_w0 * (R)cost_m(x), fma(l.x, q.y, -l.y * q.x), gsum);
           }
           emit1(gsum, 2 * i + 1, 2.0);
@@ -1133,13 +1022,8 @@ static cudaError_t launch_one(const BatchJob* jobs, int njobs, int* counter, int
   return cudaGetLastError();
 }
 
-cudaError_t launch_batched(int dtype_double, int cluster, const BatchJob* jobs, int njobs, int* counter, int mmax,
-                           cudaStream_t st, int* grid_out) {
-  if (dtype_double) {
-    if (cluster == 4) return launch_one<double, 4, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);
-    if (cluster == 2) return launch_one<double, 2, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);
-    return launch_one<double, 1, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);
-  }
+cudaError_t launch_batched(int cluster, const BatchJob* jobs, int njobs, int* counter, int mmax, cudaStream_t st,
+                           int* grid_out) {
   if (cluster == 4) return launch_one<float, 4, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);
   if (cluster == 2) return launch_one<float, 2, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);
   return launch_one<float, 1, BATCH_THREADS>(jobs, njobs, counter, mmax, st, grid_out);

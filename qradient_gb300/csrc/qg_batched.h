@@ -32,7 +32,11 @@ struct BatchC<float> {
   static constexpr int MMAX = 13;
 };
 
-cudaError_t launch_batched(int dtype_double, int cluster, const BatchJob* jobs, int njobs, int* counter, int mmax,
-                           cudaStream_t st, int* grid_out);
+cudaError_t launch_batched(int cluster, const BatchJob* jobs, int njobs, int* counter, int mmax, cudaStream_t st,
+                           int* grid_out);
+
+// The complex128 form, in 64-bit fixed point (qg_batched_fix.cu).
+cudaError_t launch_batched_fix(int cluster, const BatchJob* jobs, int njobs, int* counter, int mmax, cudaStream_t st,
+                               int* grid_out);
 
 }  // namespace qg

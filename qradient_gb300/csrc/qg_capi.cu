@@ -1470,7 +1470,10 @@ int qg_batch_launch(int dtype, const qg_batch_job* jobs, int njobs, int max_qubi
   cudaStream_t st = (cudaStream_t)stream;
   QG_CUDA(cudaMemsetAsync(ws, 0, sizeof(int), st));
   int grid = 0;
-  QG_CUDA(launch_batched(dtype == QG_C128, cluster, jobs, njobs, (int*)ws, m < 1 ? 1 : m, st, &grid));
+  if (dtype == QG_C128)
+    QG_CUDA(launch_batched_fix(cluster, jobs, njobs, (int*)ws, m < 1 ? 1 : m, st, &grid));
+  else
+    QG_CUDA(launch_batched(cluster, jobs, njobs, (int*)ws, m < 1 ? 1 : m, st, &grid));
   return QG_OK;
 }
 
