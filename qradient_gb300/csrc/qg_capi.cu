@@ -1002,6 +1002,13 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
   p.G = W.G;
   C* psi0 = (C*)(ws + W.psi);
   const int m = P.nsweeps();
+  // Overlap neighbouring sweeps (fix_bwd_kernel) where a CTA has at most four
+  // tiles: n = 21, L = 10 2.27 -> 2.10 ms; with more the overlap is a small
+  // part and the kernel with the wait at its head is the faster one (n = 24,
+  // L = 10: 14.43 against 14.54 ms; n = 22 the same).
+  bool chained = history && P.fixed;
+  for (int k = P.first_param; chained && k < m; ++k)
+    chained = ((int64_t)1 << (c->n - P.fix[k].t)) <= 4 * (int64_t)W.grid_bwd_k[k];
   for (int k = m - 1; k >= P.first_param; --k) {
     // undo, on load, the entangler the forward applied right after sweep k
     const int8_t lam_undo = k + 1 < m ? P.pre(k + 1) : P.obs_pre;
@@ -1023,12 +1030,13 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
         FixDesc d = P.fix[k];
         d.lam_undo = lam_undo;
         d.psi_undo = psi_undo;
+        d.early = k < m - 1;
         FixPtrs q = fix_ptrs(P, W, ws);
         q.psi_in = p.psi_in;
         q.psi_out = p.psi_out;
         q.lam_in = p.lam_in;
         q.lam_out = p.lam_out;
-        QG_CUDA(launch_fix_bwd(d, q, !history, W.grid_bwd_k[k], st, true));
+        QG_CUDA(launch_fix_bwd(d, q, !history, chained, W.grid_bwd_k[k], st, true));
         continue;
       }
     }

@@ -368,7 +368,15 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
 
 // ------------------------------------------------------------ backward
 
-template <int T, bool UNCOMPUTE>
+// EARLY (history mode, few tiles per CTA): what a sweep does to psi needs only
+// the forward pass, so a chain of backward sweeps brings the first tile's psi
+// into the frame before it waits for the sweep ahead of it, which lets it in
+// as it starts on its last tile (after its own wait, so that the chain is two
+// deep and everything up to the sweep before the last is complete).  n = 10,
+// L = 10: 269 -> 246 us; n = 15, L = 20: 753 -> 677; n = 17: 904 -> 824;
+// n = 18: 1068 -> 985; n = 20: 2429 -> 2265.  Triggered before the wait,
+// waiting CTAs piled up on some SMs (n = 18: 1498).
+template <int T, bool UNCOMPUTE, bool EARLY>
 __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 ? bwd_warps / (Lay<T>::NT / 32) : 1)
     fix_bwd_kernel(const __grid_constant__ FixDesc d, FixPtrs p) {
   constexpr int NT = Lay<T>::NT, NW = NT / 32;
@@ -380,7 +388,8 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
   const int ntiles = 1 << (d.n - T);
   int par = 0;
   double Tacc = 0.0, U0 = 0.0, U1 = 0.0, U2 = 0.0, gacc = 0.0;
-  pdl_wait();
+  bool early = EARLY && d.early;
+  if (!early) pdl_wait();
   const bool poison = p.flags[d.sweep] != 0;
   const int4* tab = (const int4*)(p.area + d.tab);
   const int4* ctab = (const int4*)(p.area + d.ctab);
@@ -388,6 +397,8 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const i64 x = tile_base(d, tile) | dep;
     const i64 src = (i64)ladder_fwd((uint64_t)x, masks_of(d));
+    const bool last = tile + (int)gridDim.x >= ntiles;
+    if (EARLY && last && !early) pdl_trigger();
     {
       // lambda of this tile, used once psi is in the frame; psi of the next
       const i64 y = tile_base(d, tile) | line;
@@ -404,15 +415,20 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
     for (int st = 0; st < 2; ++st) {
       i64 re[NA], im[NA];
       double2 raw[NA];
+      if (EARLY && st == 1 && early) {
+        pdl_wait();
+        early = false;
+        if (last) pdl_trigger();
+      }
       load_tile(raw, st ? p.lam_in : p.psi_in, opaque(st ? d.lam_undo : d.psi_undo), x, src, d.top, d.top_fwd);
-      if (st == 0 && opaque(d.has_gslot)) {
+      if (st == (EARLY ? 1 : 0) && opaque(d.has_gslot)) {
         // gamma of the next layer's cost: sum_x C(x) Im(conj(lam) psi), before any inverse gate
-        const double2* l = p.lam_in + x;
+        const double2* o = (EARLY ? p.psi_in : p.lam_in) + x;
         const int32_t* ci = p.cost_i + x;
 #pragma unroll
         for (int c = 0; c < NA; ++c) {
-          const double2 a = l[combine(d.top, c)];
-          gacc = fma((double)ci[combine(d.top, c)], fma(a.x, raw[c].y, -a.y * raw[c].x), gacc);
+          const double2 b = o[combine(d.top, c)], a = EARLY ? raw[c] : b, q = EARLY ? b : raw[c];
+          gacc = fma((double)ci[combine(d.top, c)], fma(a.x, q.y, -a.y * q.x), gacc);
         }
       }
       const Scale s = tile_scale<T>(raw, N, par, poison);
@@ -472,7 +488,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
         for (int c = 0; c < NA; ++c) cmul_fix<true>(re[c], im[c], __ldg(ctab + ci[combine(d.top, c)] + d.cost_maxabs));
       }
       store_tile((st ? p.lam_out : p.psi_out) + x, re, im, s, d.kout[1], d.top);
-      if (st && tile + (int)gridDim.x >= ntiles) pdl_trigger();
+      if (!EARLY && st && last) pdl_trigger();
     }
   }
   // S_j = sum_x s_j(x) w_x = T - 2 U_j over the CTA's threads
@@ -631,8 +647,9 @@ cudaError_t prepare_fix_kernels() {
       constexpr int T = decltype(tc)::value;
       const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
       cudaError_t r = cudaFuncSetAttribute(fix_fwd_kernel<T>, a, (int)fix_smem<T>(false));
-      if (r == cudaSuccess) r = cudaFuncSetAttribute(fix_bwd_kernel<T, false>, a, (int)fix_smem<T>(true));
-      if (r == cudaSuccess) r = cudaFuncSetAttribute(fix_bwd_kernel<T, true>, a, (int)fix_smem<T>(true));
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(fix_bwd_kernel<T, false, false>, a, (int)fix_smem<T>(true));
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(fix_bwd_kernel<T, true, false>, a, (int)fix_smem<T>(true));
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(fix_bwd_kernel<T, false, true>, a, (int)fix_smem<T>(true));
       return r;
     });
     if (e != cudaSuccess) return e;
@@ -714,8 +731,8 @@ int fix_ctas_per_sm(int t, bool bwd, bool uncompute) {
   const cudaError_t e = with_t(t, [&](auto tc) {
     constexpr int T = decltype(tc)::value;
     const void* fn = !bwd        ? (const void*)fix_fwd_kernel<T>
-                     : uncompute ? (const void*)fix_bwd_kernel<T, true>
-                                 : (const void*)fix_bwd_kernel<T, false>;
+                     : uncompute ? (const void*)fix_bwd_kernel<T, true, false>
+                                 : (const void*)fix_bwd_kernel<T, false, false>;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, Lay<T>::NT, fix_smem<T>(bwd));
   });
   if (e != cudaSuccess) {
@@ -739,12 +756,15 @@ cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStr
   });
 }
 
-cudaError_t launch_fix_bwd(const FixDesc& d, const FixPtrs& p, bool uncompute, int grid, cudaStream_t st, bool pdl) {
+cudaError_t launch_fix_bwd(const FixDesc& d, const FixPtrs& p, bool uncompute, bool chained, int grid,
+                           cudaStream_t st, bool pdl) {
   if (cudaError_t e = prepare_fix_kernels()) return e;
   return with_t(d.t, [&](auto tc) {
     constexpr int T = decltype(tc)::value;
-    return launch_nt(uncompute ? fix_bwd_kernel<T, true> : fix_bwd_kernel<T, false>, grid, Lay<T>::NT,
-                     fix_smem<T>(true), st, pdl, d, p);
+    return launch_nt(uncompute ? fix_bwd_kernel<T, true, false>
+                     : chained ? fix_bwd_kernel<T, false, true>
+                               : fix_bwd_kernel<T, false, false>,
+                     grid, Lay<T>::NT, fix_smem<T>(true), st, pdl, d, p);
   });
 }
 

@@ -35,6 +35,7 @@ struct FixDesc {
   int16_t kw;       // w = Xl Xq 2^-64 * 2^(pl + pq + kw)
   int8_t start, pre, lam_undo, psi_undo, periodic;
   int8_t cost, has_gslot;
+  int8_t early;             // backward, chained: the launch before this one is a chained backward sweep
   int32_t cost_maxabs, gslot;
   double cost_w0;
   int32_t slot[FIX_TMAX];  // gradient slot per active bit (from the lowest), -1 none
@@ -80,6 +81,9 @@ void fix_schedule(FixDesc& d);
 int fix_ctas_per_sm(int t, bool bwd, bool uncompute);
 cudaError_t launch_fix_tables(const FixTables& ft, const double* params, char* area, cudaStream_t st);
 cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl);
-cudaError_t launch_fix_bwd(const FixDesc& d, const FixPtrs& p, bool uncompute, int grid, cudaStream_t st, bool pdl);
+// chained: history mode, every backward sweep of the call is launched so, and d.early is
+// set on all but the first
+cudaError_t launch_fix_bwd(const FixDesc& d, const FixPtrs& p, bool uncompute, bool chained, int grid,
+                           cudaStream_t st, bool pdl);
 
 }  // namespace qg
