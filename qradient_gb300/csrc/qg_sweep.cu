@@ -926,7 +926,7 @@ struct ObsSmem {
     using C = typename C2T<R>::T;
     const size_t tile = ((size_t)1 << t) * sizeof(C);
     const size_t dvals = ((size_t)1 << t) * sizeof(R);
-    return tile + dvals + (size_t)ndiag * (sizeof(uint64_t) + sizeof(R)) + ((1 << OBS_KBITS) + 1) * sizeof(int);
+    return tile + dvals + (size_t)ndiag * (sizeof(uint64_t) + sizeof(R)) + ((1 << OBS_KBITS) + 1) * sizeof(int) + ndiag;
   }
 };
 
@@ -954,36 +954,50 @@ __global__ void __launch_bounds__(NTHREADS) observable_kernel(const __grid_const
   } else if (tid == 0) {
     offhi[0] = 0;
   }
-  if (tid == 0) {
-    int j = 0, o = 0;
-    for (int b = 0; b < n; ++b) {
-      if (j < t && d.bits[j] == b)
-        ++j;
-      else
-        outside[o++] = (uint8_t)b;
+  if (tid < n) {
+    // the bits not in the tile, ascending
+    int below = 0;
+    bool in = false;
+    for (int j = 0; j < t; ++j) {
+      below += d.bits[j] < tid;
+      in |= d.bits[j] == tid;
     }
-    if (wht) {
-      // counting sort of the diagonal terms by the k bits their mask covers
-      int cnt[(1 << OBS_KBITS) + 1] = {0};
-      auto subset = [&](const ObsTerm& tm) {
-        const uint64_t m = (1ull << tm.b0) | (tm.kind == 3 ? (1ull << tm.b1) : 0ull);
-        int sbits = 0;
-        for (int i = 0; i < kb; ++i) sbits |= (int)((m >> d.bits[8 + i]) & 1) << i;
-        return sbits;
-      };
-      for (int i = 0; i < d.ndiag; ++i) ++cnt[subset(d.term[i]) + 1];
-      for (int sb = 0; sb < (1 << OBS_KBITS); ++sb) cnt[sb + 1] += cnt[sb];
-      for (int sb = 0; sb <= (1 << OBS_KBITS); ++sb) tstart[sb] = cnt[sb];
-      for (int i = 0; i < d.ndiag; ++i) {
-        const ObsTerm& tm = d.term[i];
-        const int pos = cnt[subset(tm)]++;
-        tmask[pos] = (1ull << tm.b0) | (tm.kind == 3 ? (1ull << tm.b1) : 0ull);
-        tw[pos] = sizeof(R) == 4 ? (R)tm.wf : (R)tm.w;
+    if (!in) outside[tid - below] = (uint8_t)tid;
+  }
+  if (wht) {
+    // Order the diagonal terms by the k bits their mask covers, keeping the
+    // host's order within a subset: a term's place is the number of terms
+    // before it.  (Sorted by one thread, the pass took 23.5 us instead of
+    // 17.3 at n = 15 in complex64, 150 instead of 124 at n = 24.)
+    uint8_t* sub = (uint8_t*)(tstart + (1 << OBS_KBITS) + 1);
+    auto mask_of = [&](int i) {
+      const ObsTerm& tm = d.term[i];
+      return (1ull << tm.b0) | (tm.kind == 3 ? (1ull << tm.b1) : 0ull);
+    };
+    for (int i = tid; i < d.ndiag; i += NTHREADS) {
+      const uint64_t m = mask_of(i);
+      int sbits = 0;
+      for (int b = 0; b < kb; ++b) sbits |= (int)((m >> d.bits[8 + b]) & 1) << b;
+      sub[i] = (uint8_t)sbits;
+    }
+    __syncthreads();
+    auto weight = [&](int i) { return sizeof(R) == 4 ? (R)d.term[i].wf : (R)d.term[i].w; };
+    for (int i = tid; i < d.ndiag; i += NTHREADS) {
+      const int own = sub[i];
+      int pos = 0, next = -1;  // next: the subset's next term
+      for (int j = 0; j < d.ndiag; ++j) {
+        const int o = sub[j];
+        pos += o < own || (o == own && j < i);
+        if (o == own && j > i && next < 0) next = j;
       }
       // the last term of each run of equal weights within a subset
-      for (int sb = 0; sb < (1 << OBS_KBITS); ++sb)
-        for (int j = tstart[sb]; j < tstart[sb + 1]; ++j)
-          if (j + 1 == tstart[sb + 1] || tw[j + 1] != tw[j]) tmask[j] |= OBS_RUN_END;
+      tmask[pos] = mask_of(i) | (next < 0 || weight(next) != weight(i) ? OBS_RUN_END : 0);
+      tw[pos] = weight(i);
+    }
+    if (tid <= (1 << OBS_KBITS)) {
+      int below = 0;
+      for (int j = 0; j < d.ndiag; ++j) below += sub[j] < tid;
+      tstart[tid] = below;
     }
   }
   __syncthreads();

@@ -326,80 +326,84 @@ __device__ void sweep_setup(const SweepDesc& d, const double* params, SetupShare
   using R = decltype(C{}.x);
   const int tid = threadIdx.x;
   const int t = d.t, n = d.n;
-  if (tid < d.nxy) {
+  // The pieces go to different warps; all in the first one, they ran one after
+  // the other, longer than a sweep of a tile or two per CTA (complex64, a
+  // forward launch on its own at n = 15 15.9 -> 11.7 us; n = 20, L = 20
+  // 1.31 -> 1.20 ms).
+  //
+  // warps 0 and 1: multipliers of this sweep's rotations, scale factors of
+  // the layer's (one sine each, one copy of the code)
+  for (int i = tid; i < d.nxy + (d.has_diag ? d.nscale : 0); i += NTHREADS) {
     int f;
     double k;
-    S.u[tid] = rot_form(angle_of(d.xy[tid].a, params), &f, &k);
-    S.uf[tid] = (float)S.u[tid];
-    S.form[tid] = f;
-    S.kappa[tid] = k;
+    const double u = rot_form(angle_of(i < d.nxy ? d.xy[i].a : d.scale[i - d.nxy], params), &f, &k);
+    if (i < d.nxy) {
+      S.u[i] = u;
+      S.uf[i] = (float)u;
+      S.form[i] = f;
+      S.kappa[i] = k;
+    } else {
+      S.sc[i - d.nxy] = k;
+    }
   }
-  if (tid < d.nz) {
+  // warp 2: the Z rotations
+  if (tid >> 5 == 2) {
+    const int j = tid & 31;
     // where the Z rotation's bit lives: tile position >= 8 (a bit of the
     // element-loop index k, zk = position - 8), a bit of the thread index
     // (zk = -1), or outside the tile (zk = -2)
     int zk = -2;
-    for (int i = 0; i < t; ++i)
-      if (d.bits[i] == d.z[tid].gbit) zk = i >= 8 ? i - 8 : -1;
-    S.zk[tid] = zk;
-  }
-  if (tid == 0) {
-    int m = 0;
-    for (int j = 0; j < d.nz; ++j) {
-      int zk = -2;
-      for (int i = 8; i < t; ++i)
-        if (d.bits[i] == d.z[j].gbit) zk = i - 8;
-      if (zk >= 0) m |= 1 << zk;
+    if (j < d.nz) {
+      for (int i = 0; i < t; ++i)
+        if (d.bits[i] == d.z[j].gbit) zk = i >= 8 ? i - 8 : -1;
+      S.zk[j] = zk;
+      if (d.has_diag) {
+        sincos(0.5 * angle_of(d.z[j].a, params), &S.zs[j], &S.zc[j]);
+        S.zsf[j] = (float)S.zs[j];
+        S.zcf[j] = (float)S.zc[j];
+      }
     }
-    S.zkmask = m;
+    const unsigned m = __reduce_or_sync(0xffffffffu, zk >= 0 ? 1u << zk : 0u);
+    if (j == 0) S.zkmask = (int)m;
   }
   for (int i = tid; i < (NTHREADS / 32) * RS_N; i += NTHREADS) (&S.red[0][0])[i] = 0.0;  // clears both views
-  if (t > 8) {
-    const LadderMasks lm = ladder_masks(n, d.periodic);
-    for (int k = tid; k < (1 << (t - 8)); k += NTHREADS) {
-      S.offhi[k] = deposit((int64_t)k << 8, d.bits, t);
-      S.zpk[k] = zpattern((uint64_t)S.offhi[k], d);
-      if (ladk) ladk[k] = (int64_t)(BWD ? ladder_fwd((uint64_t)S.offhi[k], lm) : ladder_inv((uint64_t)S.offhi[k], lm));
-    }
-  } else if (tid == 0) {
-    S.offhi[0] = 0;
-    S.zpk[0] = 0;
-    if (ladk) ladk[0] = 0;
-  }
-  if (tid == 0) {
-    // bits not in the tile, ascending
-    int j = 0, o = 0;
-    for (int b = 0; b < n; ++b) {
-      if (j < t && d.bits[j] == b)
-        ++j;
-      else
-        S.outside[o++] = (uint8_t)b;
+  // warp 3: the element loop's offsets
+  if (tid >> 5 == 3) {
+    const int k = tid & 31;
+    if (t > 8) {
+      if (k < (1 << (t - 8))) {
+        const LadderMasks lm = ladder_masks(n, d.periodic);
+        S.offhi[k] = deposit((int64_t)k << 8, d.bits, t);
+        S.zpk[k] = zpattern((uint64_t)S.offhi[k], d);
+        if (ladk) ladk[k] = (int64_t)(BWD ? ladder_fwd((uint64_t)S.offhi[k], lm) : ladder_inv((uint64_t)S.offhi[k], lm));
+      }
+    } else if (k == 0) {
+      S.offhi[0] = 0;
+      S.zpk[0] = 0;
+      if (ladk) ladk[0] = 0;
     }
   }
-  if (!BWD && d.start == START_MCCLEAN && tid == 0) {
+  // warps 4 and 5: the bits not in the tile, ascending
+  if (tid >= 128 && tid - 128 < n) {
+    const int b = tid - 128;
+    int below = 0;
+    bool in = false;
+    for (int j = 0; j < t; ++j) {
+      below += d.bits[j] < b;
+      in |= d.bits[j] == b;
+    }
+    if (!in) S.outside[b - below] = (uint8_t)b;
+  }
+  // warps 6 and 7: start amplitudes by popcount
+  if (!BWD && d.start == START_MCCLEAN && tid >= 192 && tid - 192 <= n) {
     // Ry(pi/4)|0> = cos(pi/8)|0> + sin(pi/8)|1> on every qubit
+    const int k = tid - 192;
     double s8, c8;
     sincospi(0.125, &s8, &c8);
-    for (int k = 0; k <= n; ++k) {
-      double q = 1.0;
-      for (int i = 0; i < n - k; ++i) q *= c8;
-      for (int i = 0; i < k; ++i) q *= s8;
-      S.startP[k] = q;
-    }
-  }
-  // per-rotation scale factors and Z phases once per CTA, then the table
-  if (d.has_diag) {
-    for (int i = tid; i < d.nscale; i += NTHREADS) {
-      int f;
-      double k;
-      rot_form(angle_of(d.scale[i], params), &f, &k);
-      S.sc[i] = k;
-    }
-    if (tid < d.nz) {
-      sincos(0.5 * angle_of(d.z[tid].a, params), &S.zs[tid], &S.zc[tid]);
-      S.zsf[tid] = (float)S.zs[tid];
-      S.zcf[tid] = (float)S.zc[tid];
-    }
+    double q = 1.0;
+    for (int i = 0; i < n - k; ++i) q *= c8;
+    for (int i = 0; i < k; ++i) q *= s8;
+    S.startP[k] = q;
   }
   __syncthreads();
   if (d.has_diag && tid == 0) {
