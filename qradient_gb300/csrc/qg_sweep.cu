@@ -1000,7 +1000,17 @@ __global__ void __launch_bounds__(NTHREADS) observable_kernel(const __grid_const
       tstart[tid] = below;
     }
   }
-  __syncthreads();
+  // complex128 with one weight for all diagonal terms (chains, MaxCut): the
+  // transform runs on the integer sign counts, and the FP64 pipe sees one
+  // conversion and one multiply per amplitude instead of four additions and
+  // a multiply per subset (n = 24: 541 -> 283 us).  complex64 keeps its order of roundings.
+  bool one_weight = sizeof(R) == 8 && wht;
+  if (sizeof(R) == 8) {
+    for (int i = tid; i < d.ndiag; i += NTHREADS) one_weight = one_weight && d.term[i].w == d.term[0].w;
+    one_weight = __syncthreads_and(one_weight);
+  } else {
+    __syncthreads();
+  }
   pdl_trigger();
   pdl_wait();
   const int nk = tsize > NTHREADS ? tsize / NTHREADS : 1;
@@ -1022,7 +1032,28 @@ __global__ void __launch_bounds__(NTHREADS) observable_kernel(const __grid_const
         cp_async_elem(&tile[stid + k * NTHREADS], psi + (d.pre == ENT_CNOT ? ladder_inv(x, lm) : x));
       }
       cp_async_commit();
-      if (wht) {
+      if (sizeof(R) == 8 && one_weight) {
+        int b[1 << OBS_KBITS];
+#pragma unroll
+        for (int sb = 0; sb < (1 << OBS_KBITS); ++sb) {
+          int cnt = 0;
+          for (int j = tstart[sb]; j < tstart[sb + 1]; ++j) cnt += 1 - 2 * (__popcll(bd & tmask[j] & ~OBS_RUN_END) & 1);
+          b[sb] = cnt;
+        }
+#pragma unroll
+        for (int i = 0; i < OBS_KBITS; ++i)
+#pragma unroll
+          for (int k = 0; k < (1 << OBS_KBITS); ++k)
+            if (!((k >> i) & 1) && i < kb) {
+              const int u = b[k], v = b[k | (1 << i)];
+              b[k] = u + v;
+              b[k | (1 << i)] = u - v;
+            }
+        const R w = (R)d.term[0].w;
+#pragma unroll
+        for (int k = 0; k < (1 << OBS_KBITS); ++k)
+          if (k < nk) dval[k * NTHREADS + tid] = w * (R)b[k];
+      } else if (wht) {
         // the diagonal of this thread's elements while the loads land
         R b[1 << OBS_KBITS];
 #pragma unroll
