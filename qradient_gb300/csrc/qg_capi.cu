@@ -276,9 +276,10 @@ int build_layer(int n, const Layout& lay, const std::vector<LayerGate>& g, int8_
 // ------------------------------------------------------------ fixed-point sweeps (qg_fixed.cu)
 
 // complex128 circuits run on the fixed-point sweeps wherever those have an
-// instantiation: from 9 qubits on (below, a state is one tile of the double
-// kernels either way), tiles of 9..12 bits, an integer cost, and unless the
-// single-buffered double kernels are asked for.
+// instantiation: from 8 qubits on (a tile of fewer is less than a warp of
+// eight amplitudes a thread; n = 8, L = 10: 316 us in the double kernels, 204
+// here), tiles of 8..12 bits, an integer cost, and unless the single-buffered
+// double kernels are asked for.
 bool fixed_path(const qg_circuit* c, int dtype) {
   if (dtype != QG_C128 || c->n < FIX_TMIN || c->L < 1) return false;
   if (c->kind == 1 && c->cost_kind != COST_INT) return false;

@@ -619,6 +619,8 @@ size_t fix_smem(bool bwd) {
 template <typename F>
 cudaError_t with_t(int t, F f) {
   switch (t) {
+    case 8:
+      return f(std::integral_constant<int, 8>());
     case 9:
       return f(std::integral_constant<int, 9>());
     case 10:

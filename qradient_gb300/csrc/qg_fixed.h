@@ -7,7 +7,7 @@
 
 namespace qg {
 
-constexpr int FIX_TMIN = 9, FIX_TMAX = 12;  // tile bits with an instantiation
+constexpr int FIX_TMIN = 8, FIX_TMAX = 12;  // tile bits with an instantiation
 // A thread holds 2^FIX_E amplitudes.  With 16 instead of 8 a layer has fewer
 // exchanges, but twice the registers halve the resident warps and the code no
 // longer fits the instruction cache: n = 24, L = 20 31.3 against 28.9 ms.

@@ -13,7 +13,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,L,ent,place", [(9, 40, "cnot", "before"), (12, 30, "cz", "after"), (13, 30, "cnot", "after"),
+@pytest.mark.parametrize("n,L,ent,place", [(8, 40, "cz", "before"), (9, 40, "cnot", "before"), (12, 30, "cz", "after"), (13, 30, "cnot", "after"),
                                            (17, 20, "cnot", "before"), (19, 10, None, "before"),
                                            (20, 8, "cnot_periodic", "before"), (21, 5, "cnot", "before")])
 def test_mcclean(n, L, ent, place):

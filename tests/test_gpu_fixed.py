@@ -1,7 +1,7 @@
 """The fixed-point complex128 sweeps (qg_fixed.cu) against the oracle.
 
 One case per sweep layout the default rule takes (single tile, two sweeps of
-9..12-bit tiles, three sweeps), every tuned tile size with a remainder, and
+8..12-bit tiles, three sweeps), every tuned tile size with a remainder, and
 the states whose tiles leave the usual range: zero tiles, tiny, huge and
 non-finite amplitudes.  Tolerance: the oracle's own double rounding, 1e-12
 normwise, as in the other complex128 tests (a tile's fixed-point step is
@@ -47,12 +47,12 @@ def _check(n, L, ent="cnot", place="before", seed=0, axes=None, ini=None, tile=0
     assert abs(c.run_expec_val(ini_state=start) - E0) <= TOL * max(scale ** 2, abs(E0))
 
 
-@pytest.mark.parametrize("n", [9, 10, 11, 12, 13, 16, 17, 18, 19, 20, 21, 22])
+@pytest.mark.parametrize("n", [8, 9, 10, 11, 12, 13, 16, 17, 18, 19, 20, 21, 22])
 def test_default_layouts(n):
     _check(n, 3 if n < 18 else 2, ("cnot", "cz", None)[n % 3], ("before", "after")[n % 2])
 
 
-@pytest.mark.parametrize("tile,n", [(9, 9), (9, 14), (9, 16), (10, 17), (10, 19), (11, 15), (11, 20), (12, 13), (12, 21)])
+@pytest.mark.parametrize("tile,n", [(8, 8), (8, 11), (8, 15), (9, 9), (9, 14), (9, 16), (10, 17), (10, 19), (11, 15), (11, 20), (12, 13), (12, 21)])
 def test_tuned_tiles(tile, n):
     _check(n, 2, "cnot" if n % 2 else "cnot_periodic", "before", seed=tile, tile=tile)
 
@@ -60,7 +60,7 @@ def test_tuned_tiles(tile, n):
 @pytest.mark.parametrize("axis", [0, 1, 2])
 def test_one_axis(axis):
     """Every bit a butterfly level (X, Y), or none (Z)."""
-    for n in (9, 11, 12, 13, 19):
+    for n in (8, 9, 11, 12, 13, 19):
         _check(n, 2, "cnot", "after", axes=axis)
 
 
