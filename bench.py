@@ -10,18 +10,20 @@ layer.  A step is one full grad_run (E and all L*n gradients).
 value      circuits/s over the timed steps with inputs resident on the device
 e2e        the same through the public API (McClean.grad_run) with host
            angles in (H2D) and host E + gradient out (D2H) every step
-roofline   dominant kernel (the backward sweep): FP64-bound on GB300.  The
-           achieved rate counts the FP64 instructions the kernel executes
-           (ncu counts of the same workload, profiles/backward_sweep_traffic.json)
-           against GB300's FP64 issue rate at the SM clock sampled during the
-           timed region; the HBM view and the step-level T_roof / T_measured
-           are reported beside it
+roofline   dominant kernel (the backward sweep): the bytes it cannot do
+           without (psi and lambda read, lambda written) over its mean
+           duration, against the measured HBM bandwidth.  Neither precision
+           reaches it: complex128 sweeps are bound by instruction issue
+           (64-bit fixed-point arithmetic; the counters beside it are ncu's,
+           profiles/backward_sweep_traffic.json), complex64 ones by
+           shared-memory instructions and latency.  The step-level
+           T_roof / T_measured is reported beside it
 cpu_baseline  the CPU oracle (C + OpenMP restatement of the reference's
            numpy algorithm) on the host cores, on a bounded sample
 --impl reference  times that CPU restatement as the reference arm
 
 The default run adds, measured in the same process after the headline:
-  c64        the same circuit in complex64 (HBM-bound), with its HBM fraction
+  c64        the same circuit in complex64, with its HBM fraction
   cz_after   the same circuit with the CZ ladder after the rotations
   qaoa       QAOA MaxCut n=24 p=10 complex128
   large      McClean n=28 L=50 complex128 (its state history does not fit in
@@ -176,12 +178,6 @@ def measured_peaks():
             return json.load(f)
     except (OSError, ValueError):
         return {}
-
-
-# GB300 FP64: 2 FMA lanes per SM per clock (a warp's DFMA holds the pipe for
-# 16 cycles), 152 SMs; 4 flops per SM per clock counting an FMA as 2
-GB300_SMS = 152
-FP64_FLOPS_PER_SM_CLK = 4
 
 
 def cpu_info():
@@ -589,24 +585,16 @@ def run_serving(args):
         print(json.dumps(line))
 
 
-def executed_fp64(dtype, n, L, seed):
-    """Executed FP64 work of the headline workload per grad_run, from the ncu
-    capture summarised in profiles/backward_sweep_traffic.json: per kernel
-    class, the DFMA / DMUL / DADD thread instructions of every launch of one
-    grad_run (flops = 2 DFMA + DMUL + DADD), and the DRAM bytes per backward
-    launch.  None when the capture does not match the workload."""
+def backward_profile(dtype, n):
+    """ncu's figures of a backward sweep launch of the headline workload
+    (profiles/backward_sweep_traffic.json): DRAM bytes and, for complex128,
+    the issue and pipe activity.  Empty when the capture is of another size."""
     tpath = os.path.join(ROOT, "profiles", "backward_sweep_traffic.json")
     try:
         prof = json.load(open(tpath)).get(dtype) or {}
     except (OSError, ValueError):
-        return None
-    if prof.get("n") != n:
-        return None
-    ex = prof.get("executed_fp64") or {}
-    if ex.get("layers") != L or ex.get("seed") != seed:
-        ex = {}
-    return {"traffic": prof.get("dram_bytes_per_launch"), "pipe_busy": prof.get("fp64_pipe_busy_ncu"),
-            "executed": ex}
+        return {}
+    return prof if prof.get("n") == n else {}
 
 
 def main():
@@ -727,49 +715,20 @@ def main():
     achieved_gbs = per_launch_bytes / bwd_avg_s * 1e-9 if bwd_n else None
     peaks = measured_peaks()
     hbm_peak = peaks.get("hbm_gbs", 6800.0)
-    prof = executed_fp64(args.dtype, args.n, args.layers, args.seed) or {}
-    ex = prof.get("executed") or {}
+    prof = backward_profile(args.dtype, args.n)
     share = {k: v[0] / ms_prof for k, v in kinfo.items()}
+    t_roof_ms = B / (hbm_peak * 1e9) * 1e3
+    roof = {"bound": "hbm",
+            "kernel": "fix_bwd_kernel" if args.dtype == "complex128" else "sweep_bwd_kernel<float,history,12>",
+            "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
+            "frac": achieved_gbs / hbm_peak if achieved_gbs else None,
+            "traffic": prof.get("dram_bytes_per_launch"), "peak_source": "MEASURED_PEAKS.json hbm_gbs",
+            "step": {"t_roof_ms": t_roof_ms, "t_measured_ms": ms_per_step, "frac": t_roof_ms / ms_per_step,
+                     "algorithmic_bytes": B},
+            "launch_ms_avg": bwd_avg_s * 1e3, "launches": bwd_n, "kernel_share": share}
     if args.dtype == "complex128":
-        sm_mhz = clk.get("sm_mhz") or peaks.get("sm_max_mhz", 2070.0)
-        fp64_peak = FP64_FLOPS_PER_SM_CLK * GB300_SMS * sm_mhz * 1e6 * 1e-12  # TFLOP/s
-        bex = ex.get("backward") or {}
-        fex = ex.get("forward") or {}
-        achieved = None
-        if bex.get("flops") and bwd_n:
-            achieved = bex["flops"] / bex["launches"] / bwd_avg_s * 1e-12
-        # step level: the binding roof of the whole grad_run
-        step_flops = (bex.get("flops") or 0) + (fex.get("flops") or 0) + ((ex.get("other") or {}).get("flops") or 0)
-        t_roof_ms = max(B / (hbm_peak * 1e9), step_flops / (fp64_peak * 1e12)) * 1e3 if step_flops else None
-        roof = {"bound": "fp64", "kernel": "sweep_bwd_kernel<double,history,11>", "achieved": achieved,
-                "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak if achieved else None,
-                "traffic": prof.get("traffic"),
-                "peak_source": "GB300 FP64 issue rate: 2 DFMA lanes per SM per clock (4 flops) x 152 SMs x the "
-                               "median SM clock sampled during the timed region (%.0f MHz)" % sm_mhz,
-                "achieved_source": "FP64 flops the backward launches execute (2 DFMA + DMUL + DADD thread "
-                                   "instructions, ncu, every backward launch of one grad_run of this workload: "
-                                   "profiles/backward_sweep_traffic.json) / their mean duration (CUDA events "
-                                   "around every launch on the launching stream)",
-                "fp64_pipe_busy_ncu": prof.get("pipe_busy"),
-                # the credited algorithmic count (6 flops per rotation as the
-                # reference's gate formula writes it, 4 per reduction, per
-                # amplitude) at the same duration, for reference
-                "algorithmic_rate_tflops": (2 ** args.n) * args.n * (4 + 6) * args.layers / bwd_per_step /
-                                           bwd_avg_s * 1e-12 if bwd_n else None,
-                "hbm": {"achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
-                        "frac": achieved_gbs / hbm_peak if achieved_gbs else None,
-                        "peak_source": "MEASURED_PEAKS.json hbm_gbs"},
-                "step": {"t_roof_ms": t_roof_ms, "t_measured_ms": ms_per_step,
-                         "frac": t_roof_ms / ms_per_step if t_roof_ms else None,
-                         "executed_fp64_flops": step_flops or None, "algorithmic_bytes": B},
-                "launch_ms_avg": bwd_avg_s * 1e3, "launches": bwd_n, "kernel_share": share}
-    else:
-        roof = {"bound": "hbm", "kernel": "sweep_bwd_kernel<float,history,12>", "achieved": achieved_gbs,
-                "peak": hbm_peak, "unit": "GB/s", "frac": achieved_gbs / hbm_peak if achieved_gbs else None,
-                "traffic": prof.get("traffic"), "peak_source": "MEASURED_PEAKS.json hbm_gbs",
-                "step": {"t_roof_ms": B / (hbm_peak * 1e9) * 1e3, "t_measured_ms": ms_per_step,
-                         "frac": B / (hbm_peak * 1e9) * 1e3 / ms_per_step, "algorithmic_bytes": B},
-                "launch_ms_avg": bwd_avg_s * 1e3, "launches": bwd_n, "kernel_share": share}
+        roof["issue_active_ncu"] = prof.get("issue_active_ncu")
+        roof["fp64_pipe_busy_ncu"] = prof.get("fp64_pipe_busy_ncu")
 
     launches_per_step = (fwd_n + bwd_n + kinfo["observable"][1]) / args.steps + 1  # + the finalize kernel
     line = {

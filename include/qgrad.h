@@ -143,19 +143,20 @@ int qg_sample(int n, int dtype, const void* state_dev, int64_t nshots, uint64_t 
  * amplitudes in shared memory and applies every rotation on those bits in
  * one pass (the fusion depth); ctas_per_sm sets the persistent grid (block
  * shape across the SMs, capped at what fits).  0 restores the default
- * (tile_bits 11 for complex128, 12 for complex64; complex128 takes 12 for
- * the first sweep of a layer where that saves a sweep per layer, with 11
- * for the others where that costs none; ctas_per_sm from the
+ * (complex64: tile_bits 12; complex128: sweep sizes chosen by qubit count,
+ * 8 to 12 bits; ctas_per_sm from the
  * occupancy query).  A non-zero tile_bits applies to every sweep.
  * tile_bits: 5..12 for complex128, 6..13 for
  * complex64 (the backward sweep holds two tiles in shared memory); tiles
  * larger than the state use the whole state.  Call before launches that use the handle, not while
  * another thread uses it; the workspace size may change with the setting.
  * flags: QG_TUNE_FWD_PIPELINED or QG_TUNE_FWD_PLAIN choose the forward
- * sweep kernel (0: the default, pipelined).
- * qg_get_tuning reports the effective values (tile bits of a layer's first
- * sweep after clamping to n, CTAs per SM of the backward sweeps, the
- * forward kernel flag).  The autotuner of
+ * sweep kernel (0: the default, pipelined).  complex128 sweeps of 8 bits or
+ * more run in 64-bit fixed point, which has one forward kernel;
+ * QG_TUNE_FWD_PLAIN and tile_bits 5..7 select the double sweeps.
+ * qg_get_tuning reports the effective values (tile bits after clamping to n,
+ * for a default complex128 handle those of the double sweeps; CTAs per SM of
+ * the backward sweeps; the forward kernel flag).  The autotuner of
  * qradient_gb300/tuning.py picks them by timing. */
 enum {
   QG_TUNE_FWD_PIPELINED = 1, /* forward sweeps prefetch the next tile (double-buffered) */
@@ -217,8 +218,8 @@ int qg_plateau_step(double* params_dev, const double* grad_dev, int nparams, con
 
 /* ---- Batched persistent execution (no reference counterpart: the
  * reference runs one circuit per Python call).  Many small circuits, each
- * a whole run or grad_run with psi and lambda resident in shared memory,
- * in one launch (CUDA-graph capturable).  Limits: complex64 n <= 15,
+ * a whole run or grad_run with psi and lambda resident in shared memory
+ * (complex64) or registers (complex128), in one launch (CUDA-graph capturable).  Limits: complex64 n <= 15,
  * complex128 n <= 14, L <= 4096, and for QAOA an integer cost with
  * |m| <= 511. */
 typedef struct qg_term {
@@ -277,8 +278,9 @@ int qg_batch_launch(int dtype, const qg_batch_job* jobs_dev, int njobs, int max_
  * may synchronise the device) after start-up.  Same inputs and outputs as
  * qg_grad in uncompute mode, but the scratch is a library-owned static
  * device array of QG_NOALLOC_SCRATCH_BYTES that every GPU loading the
- * library's device code holds until exit.  Circuits whose uncompute
- * workspace exceeds it get QG_ERR_UNSUPPORTED.  The first call on a device
+ * library's device code holds until exit.  Circuits whose smallest uncompute
+ * workspace (complex128: without the fixed-point sweeps' phase tables) exceeds
+ * it get QG_ERR_UNSUPPORTED.  The first call on a device
  * looks up the array's address (with that device current) and caches it; a
  * context reset (cudaDeviceReset) invalidates the cached address, so the
  * entry point must not be used after one.  Calls share the array and it

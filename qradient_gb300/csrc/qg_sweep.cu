@@ -7,6 +7,12 @@
 //   observable         physical_components/observable.py:34-73, base.py:17-20
 //   McClean grad_run   circuit_logic/mc_clean.py:47-78
 //   QAOA grad_run      circuit_logic/qaoa.py:40-70
+//
+// complex64 circuits run here, and of the complex128 ones those that the
+// fixed-point sweeps (qg_fixed.cu) do not take: fewer than eight qubits, no
+// layers, a real-valued cost, tiles tuned to 5-7 bits, single-buffered forward
+// sweeps asked for, or a workspace without room for phase tables.  The
+// observable pass and the finaliser serve both.
 #include <atomic>
 #include <mutex>
 

@@ -234,7 +234,7 @@ class Server:
     def _launch_small(self, reqs):
         # one batch per dtype and cluster size, each on the next batch stream:
         # the launches of a round overlap instead of queueing behind the
-        # longest (4-CTA complex128 jobs, FP64-bound, run longest)
+        # longest (4-CTA complex128 jobs run longest)
         by_key = collections.defaultdict(list)
         for r in reqs:
             n = r.circuit.qnum
