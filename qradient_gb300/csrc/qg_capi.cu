@@ -382,6 +382,15 @@ void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
   const int layers = c->L + ini;
   FixTables& f = P.ft;
   memset(&f, 0, sizeof f);
+  // Amplitudes a thread.  Up to 17 qubits an SM has one or two tiles and a
+  // sweep lasts as long as a warp's own instructions: with four, half of them
+  // (n = 12, L = 20: 603 -> 489 us; n = 15: 662 -> 546; n = 17: 817 -> 763;
+  // n = 18, with more warps than the chip can issue for, 976 -> 1307).  One
+  // tile of 10 or 11 bits has the warps already, and fewer stages with eight
+  // (n = 10, L = 10: 237 against 247 us; n = 11: 309 against 415).
+  f.e = n <= 17 && (per > 1 || n < 10) ? 2 : FIX_E;
+  for (const FixSweep& s : lay)
+    if (s.t > FIX_TMAX2) f.e = FIX_E;
   f.n = n;
   f.per_layer = per;
   f.ini_layers = ini;
@@ -396,7 +405,7 @@ void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
     f.nact[s] = lay[s].k;
     f.lo[s] = lay[s].lo;
     f.off[s] = f.layer_bytes;
-    f.layer_bytes += fix_table_entries(lay[s].t, lay[s].k) * 16;
+    f.layer_bytes += fix_table_entries(lay[s].t, lay[s].k, f.e) * 16;
   }
   f.ctab_bytes = f.cost == COST_INT ? (2 * (int64_t)f.cost_maxabs + 1) * 16 : 0;
   auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
@@ -418,15 +427,16 @@ void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
       d.n = n;
       d.t = lay[s].t;
       d.nact = lay[s].k;
-      d.nst = fix_stages(lay[s].k);
+      d.e = f.e;
+      d.nst = fix_stages(lay[s].k, f.e);
       const int low = d.t - lay[s].k;
       d.low = low;
       d.lo = lay[s].lo;
       const LadderMasks lm = ladder_masks(n, P.periodic);
       d.odd = lm.odd;
       d.even = lm.even;
-      for (int b = 0; b < FIX_E; ++b) {
-        const int j = d.t - FIX_E + b;  // local bit
+      for (int b = 0; b < d.e; ++b) {
+        const int j = d.t - d.e + b;  // local bit
         d.top[b] = (int64_t)1 << (j < low ? j : lay[s].lo + j - low);
         d.top_fwd[b] = (int64_t)ladder_fwd((uint64_t)d.top[b], lm);
         d.top_inv[b] = (int64_t)ladder_inv((uint64_t)d.top[b], lm);
@@ -437,7 +447,7 @@ void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
         const int axis = li < 0 ? AX_Y : mc ? c->axes[(size_t)li * n + q] : AX_X;
         if (li >= 0) d.slot[a] = mc ? li * n + q : li * (n + 1) + q;
         // the stage and in-thread bit that hold local bit j
-        const int st = (d.t - 1 - j) / FIX_E, lo = d.t - FIX_E * (st + 1);
+        const int st = (d.t - 1 - j) / d.e, lo = d.t - d.e * (st + 1);
         const int cb = lo >= 0 ? j - lo : j;
         d.code[st] |= (uint8_t)((axis == AX_X ? 1 : axis == AX_Y ? 2 : 0) << (2 * cb));
       }
@@ -628,7 +638,7 @@ WsLayout ws_layout(const qg_circuit* c, int dtype, int op, const Program& P) {
   if (P.fixed) {
     for (const auto& d : P.fix) {
       const int64_t nt = (int64_t)1 << (n - d.t);
-      int pf = fix_ctas_per_sm(d.t, false, unc), pb = fix_ctas_per_sm(d.t, true, unc);
+      int pf = fix_ctas_per_sm(d, false, unc), pb = fix_ctas_per_sm(d, true, unc);
       if (tuned > 0) pf = std::min(pf, tuned), pb = std::min(pb, tuned);
       w.grid_fwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pf));
       w.grid_bwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pb));

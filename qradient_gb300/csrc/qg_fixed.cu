@@ -61,15 +61,12 @@ __device__ __forceinline__ void exchange(unsigned char* ex, i64* re, i64* im) {
   }
 }
 // between the neighbouring stages s-1 and s (UP: to s)
-template <int T, bool UP>
+template <int T, bool UP, int S = 1>
 __device__ __forceinline__ void exchange_at(unsigned char* ex, i64* re, i64* im, int s) {
-  constexpr int N = Lay<T>::NS;
-  if (s == 1)
-    exchange<T, UP ? 0 : 1, UP ? 1 : 0>(ex, re, im);
-  else if (N == 3 || s == 2)
-    exchange<T, UP ? 1 : 2, UP ? 2 : 1>(ex, re, im);
-  else if constexpr (N > 3)
-    exchange<T, UP ? 2 : 3, UP ? 3 : 2>(ex, re, im);
+  if (S == Lay<T>::NS - 1 || s == S)
+    exchange<T, UP ? S - 1 : S, UP ? S : S - 1>(ex, re, im);
+  else if constexpr (S < Lay<T>::NS - 1)
+    exchange_at<T, UP, S + 1>(ex, re, im, s);
 }
 
 // ------------------------------------------------------------ stages
@@ -120,7 +117,7 @@ __device__ __forceinline__ void phase_mul(i64* re, i64* im, const int4* tab, int
 // ------------------------------------------------------------ addresses
 
 // element offset of in-thread index c from the offsets of its bits
-__device__ __forceinline__ i64 combine(const int64_t (&o)[E], int c) {
+__device__ __forceinline__ i64 combine(const int64_t (&o)[FIX_E], int c) {
   i64 x = 0;
 #pragma unroll
   for (int i = 0; i < E; ++i)
@@ -149,7 +146,7 @@ __device__ __forceinline__ LadderMasks masks_of(const FixDesc& d) {
 // the images of its parts (`src`: that of tile and thread, `top` those of the
 // in-thread bits).
 __device__ __forceinline__ void load_tile(double2* raw, const double2* v, int ent, i64 x, i64 src,
-                                          const int64_t (&top)[E], const int64_t (&ltop)[E]) {
+                                          const int64_t (&top)[FIX_E], const int64_t (&ltop)[FIX_E]) {
   if (ent == ENT_CNOT) {
 #pragma unroll
     for (int c = 0; c < NA; ++c) raw[c] = v[src ^ combine(ltop, c)];
@@ -289,7 +286,7 @@ __device__ __forceinline__ double2 unscale(int q) {
 
 // results of stage 0's layout to memory
 __device__ __forceinline__ void store_tile(double2* out, const i64* re, const i64* im, const Scale& s, int kout,
-                                           const int64_t (&top)[E]) {
+                                           const int64_t (&top)[FIX_E]) {
   const int k = -(s.p + kout);
   if (s.q == 0) {
 #pragma unroll
@@ -303,12 +300,11 @@ __device__ __forceinline__ void store_tile(double2* out, const i64* re, const i6
 }
 
 // Prefetch into L2 the 128-byte lines of a tile, one of eight amplitudes per
-// thread (their images under the ladder share a line as well).  Backward
+// thread, or two threads to a line (their images under the ladder share a line as well).  Backward
 // only: 309 -> 302 us per sweep at n = 24; the forward sweeps lost 3%.
 template <int T>
 __device__ __forceinline__ i64 line_index(const FixDesc& d) {
-  static_assert(E == 3, "one line per thread");
-  const int t = threadIdx.x << 3;
+  const int t = threadIdx.x << E;
   return (i64)(t & ((1 << d.low) - 1)) | (i64)(t >> d.low) << d.lo;
 }
 __device__ __forceinline__ void prefetch_line(const double2* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -534,6 +530,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
   }
 }
 
+#if QG_FIX_E == 3
 // ------------------------------------------------------------ phase tables
 //
 // One launch per run / grad_run fills the tables of every sweep (one CTA per
@@ -582,10 +579,11 @@ __global__ void __launch_bounds__(256) fix_tables_kernel(const __grid_constant__
       (half ? hi : lo)[e] = v;
     }
     __syncthreads();
-    const int nst = fix_stages(k), skip = fix_table_skip(T, k);
+    const int E = f.e;
+    const int nst = fix_stages(k, E), skip = fix_table_skip(T, k, E);
     const int lw = T - E - skip;
     int4* tab = (int4*)(area + f.tab0 + layer * f.layer_bytes + f.off[s]);
-    for (int i = tid; i < (NA << lw); i += 256) {
+    for (int i = tid; i < (1 << (E + lw)); i += 256) {
       const int c = i >> lw, th = (i & ((1 << lw) - 1)) << skip;
       // local index of (th, c) in the last stage's layout
       const int low = T - E * nst, r = E + low;
@@ -610,6 +608,7 @@ __global__ void __launch_bounds__(256) fix_tables_kernel(const __grid_constant__
     if (tid == 0) flags[sweep] = bad;
   }
 }
+#endif
 
 template <int T>
 size_t fix_smem(bool bwd) {
@@ -618,6 +617,8 @@ size_t fix_smem(bool bwd) {
 
 template <typename F>
 cudaError_t with_t(int t, F f) {
+  // 4 amplitudes a thread: up to FIX_TMAX2
+  if (QG_FIX_E == 2 && t > FIX_TMAX2) return cudaErrorInvalidValue;
   switch (t) {
     case 8:
       return f(std::integral_constant<int, 8>());
@@ -625,10 +626,12 @@ cudaError_t with_t(int t, F f) {
       return f(std::integral_constant<int, 9>());
     case 10:
       return f(std::integral_constant<int, 10>());
+#if QG_FIX_E == 3
     case 11:
       return f(std::integral_constant<int, 11>());
     case 12:
       return f(std::integral_constant<int, 12>());
+#endif
   }
   return cudaErrorInvalidValue;
 }
@@ -644,7 +647,7 @@ cudaError_t prepare_fix_kernels() {
   if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
   if (ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
   std::lock_guard<std::mutex> lock(mu);
-  for (int t = FIX_TMIN; t <= FIX_TMAX; ++t) {
+  for (int t = FIX_TMIN; t <= (QG_FIX_E == 3 ? FIX_TMAX : FIX_TMAX2); ++t) {
     e = with_t(t, [](auto tc) {
       constexpr int T = decltype(tc)::value;
       const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -678,6 +681,51 @@ cudaError_t launch_nt(void (*kern)(D, P), int grid, int nt, size_t smem, cudaStr
 
 }  // namespace
 
+#define FIXFN2(f, e) f##_e##e
+#define FIXFN1(f, e) FIXFN2(f, e)
+#define FIXFN(f) FIXFN1(f, QG_FIX_E)
+
+int FIXFN(fix_ctas_per_sm)(int t, bool bwd, bool uncompute) {
+  int blocks = 0;
+  if (prepare_fix_kernels() != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  const cudaError_t e = with_t(t, [&](auto tc) {
+    constexpr int T = decltype(tc)::value;
+    const void* fn = !bwd        ? (const void*)fix_fwd_kernel<T>
+                     : uncompute ? (const void*)fix_bwd_kernel<T, true, false>
+                                 : (const void*)fix_bwd_kernel<T, false, false>;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, Lay<T>::NT, fix_smem<T>(bwd));
+  });
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return blocks > 0 ? blocks : 1;
+}
+
+cudaError_t FIXFN(launch_fix_fwd)(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl) {
+  if (cudaError_t e = prepare_fix_kernels()) return e;
+  return with_t(d.t, [&](auto tc) {
+    constexpr int T = decltype(tc)::value;
+    return launch_nt(fix_fwd_kernel<T>, grid, Lay<T>::NT, fix_smem<T>(false), st, pdl, d, p);
+  });
+}
+
+cudaError_t FIXFN(launch_fix_bwd)(const FixDesc& d, const FixPtrs& p, bool uncompute, bool chained, int grid,
+                                  cudaStream_t st, bool pdl) {
+  if (cudaError_t e = prepare_fix_kernels()) return e;
+  return with_t(d.t, [&](auto tc) {
+    constexpr int T = decltype(tc)::value;
+    return launch_nt(uncompute ? fix_bwd_kernel<T, true, false>
+                     : chained ? fix_bwd_kernel<T, false, true>
+                               : fix_bwd_kernel<T, false, false>,
+                     grid, Lay<T>::NT, fix_smem<T>(true), st, pdl, d, p);
+  });
+}
+
+#if QG_FIX_E == 3
 // The scaling of a sweep, from the number of its butterfly levels alone.  h
 // counts half bits of the tile's norm above 2^60: a level adds one, a phase
 // product takes eight (its table is scaled by 2^60), the cost product four
@@ -690,7 +738,7 @@ void fix_schedule(FixDesc& d) {
   int m[FIX_STAGES] = {};
   int levels = 0;
   for (int s = 0; s < d.nst; ++s) {
-    for (int i = 0; i < E; ++i) m[s] += ((d.code[s] >> (2 * i)) & 3) != 0;
+    for (int i = 0; i < FIX_E; ++i) m[s] += ((d.code[s] >> (2 * i)) & 3) != 0;
     levels += m[s];
   }
   for (int dir = 0; dir < 2; ++dir) {
@@ -724,50 +772,28 @@ void fix_schedule(FixDesc& d) {
   }
 }
 
-int fix_ctas_per_sm(int t, bool bwd, bool uncompute) {
-  int blocks = 0;
-  if (prepare_fix_kernels() != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
-  const cudaError_t e = with_t(t, [&](auto tc) {
-    constexpr int T = decltype(tc)::value;
-    const void* fn = !bwd        ? (const void*)fix_fwd_kernel<T>
-                     : uncompute ? (const void*)fix_bwd_kernel<T, true, false>
-                                 : (const void*)fix_bwd_kernel<T, false, false>;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, Lay<T>::NT, fix_smem<T>(bwd));
-  });
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
-  return blocks > 0 ? blocks : 1;
-}
-
 cudaError_t launch_fix_tables(const FixTables& f, const double* params, char* area, cudaStream_t st) {
   const int grid = f.nsweeps < 1 ? 1 : f.nsweeps < 1024 ? f.nsweeps : 1024;
   fix_tables_kernel<<<grid, 256, 0, st>>>(f, params, area);
   return cudaGetLastError();
 }
 
-cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl) {
-  if (cudaError_t e = prepare_fix_kernels()) return e;
-  return with_t(d.t, [&](auto tc) {
-    constexpr int T = decltype(tc)::value;
-    return launch_nt(fix_fwd_kernel<T>, grid, Lay<T>::NT, fix_smem<T>(false), st, pdl, d, p);
-  });
-}
+// 8 or 4 amplitudes a thread (qg_fixed2.cu)
+int fix_ctas_per_sm_e2(int t, bool bwd, bool uncompute);
+cudaError_t launch_fix_fwd_e2(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl);
+cudaError_t launch_fix_bwd_e2(const FixDesc& d, const FixPtrs& p, bool uncompute, bool chained, int grid,
+                              cudaStream_t st, bool pdl);
 
+int fix_ctas_per_sm(const FixDesc& d, bool bwd, bool uncompute) {
+  return (d.e == 2 ? fix_ctas_per_sm_e2 : fix_ctas_per_sm_e3)(d.t, bwd, uncompute);
+}
+cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl) {
+  return (d.e == 2 ? launch_fix_fwd_e2 : launch_fix_fwd_e3)(d, p, grid, st, pdl);
+}
 cudaError_t launch_fix_bwd(const FixDesc& d, const FixPtrs& p, bool uncompute, bool chained, int grid,
                            cudaStream_t st, bool pdl) {
-  if (cudaError_t e = prepare_fix_kernels()) return e;
-  return with_t(d.t, [&](auto tc) {
-    constexpr int T = decltype(tc)::value;
-    return launch_nt(uncompute ? fix_bwd_kernel<T, true, false>
-                     : chained ? fix_bwd_kernel<T, false, true>
-                               : fix_bwd_kernel<T, false, false>,
-                     grid, Lay<T>::NT, fix_smem<T>(true), st, pdl, d, p);
-  });
+  return (d.e == 2 ? launch_fix_bwd_e2 : launch_fix_bwd_e3)(d, p, uncompute, chained, grid, st, pdl);
 }
+#endif
 
 }  // namespace qg

@@ -11,14 +11,18 @@ constexpr int FIX_TMIN = 8, FIX_TMAX = 12;  // tile bits with an instantiation
 // A thread holds 2^FIX_E amplitudes.  With 16 instead of 8 a layer has fewer
 // exchanges, but twice the registers halve the resident warps and the code no
 // longer fits the instruction cache: n = 24, L = 20 31.3 against 28.9 ms.
-constexpr int FIX_E = 3;
-constexpr int FIX_STAGES = (FIX_TMAX + FIX_E - 1) / FIX_E;
+// With 4 a circuit of few tiles has twice the warps to hide the latency of
+// dependent instructions behind (see build_fixed, which chooses); those are
+// the instantiations of up to FIX_TMAX2 tile bits in qg_fixed2.cu.
+constexpr int FIX_E = 3, FIX_TMAX2 = 10;
+constexpr int FIX_STAGES = (FIX_TMAX + 1) / 2;
 
 // One sweep: every rotation on the tile's active bits (its top `nact` local
 // bits), each as V D V^-1 with V the Clifford that turns the rotation's Pauli
-// into Z.  Bits are handled in stages of FIX_E local bits from the top.
+// into Z.  Bits are handled in stages of e local bits from the top.
 struct FixDesc {
   int32_t n, t, nact, nst;  // qubits, tile bits, active bits, stages
+  int32_t e;                // in-thread bits: FIX_E or 2
   // The tile's local bits: [0, low) are the same global bits, [low, t) the
   // active ones, global [lo, lo + t - low).  Element offsets of the top
   // FIX_E local bits, and their images under the CNOT ladder and its inverse.
@@ -45,6 +49,7 @@ struct FixDesc {
 
 // What the table kernel needs of a whole circuit.
 struct FixTables {
+  int32_t e;                                  // in-thread bits of every sweep
   int32_t n, nsweeps, per_layer, ini_layers;  // ini_layers: leading layers of fixed Ry(pi/4)
   int32_t kind, nparams;                      // 0 McClean, 1 QAOA
   int32_t t[QMAX], nact[QMAX], lo[QMAX];      // per sweep of a layer: tile bits, active bits, lowest active bit
@@ -67,18 +72,18 @@ struct FixPtrs {
   int32_t G;
 };
 
-__host__ __device__ inline int fix_stages(int nact) { return nact <= 0 ? 1 : (nact + FIX_E - 1) / FIX_E; }
+__host__ __device__ inline int fix_stages(int nact, int e) { return nact <= 0 ? 1 : (nact + e - 1) / e; }
 // Phase-table entries of a sweep: [in-thread index][thread index of the last
 // stage's layout without its low bits, which are inactive unless that stage
 // reaches the lowest bits].
-__host__ __device__ inline int fix_table_skip(int t, int nact) {
-  const int lo = t - FIX_E * fix_stages(nact);
+__host__ __device__ inline int fix_table_skip(int t, int nact, int e) {
+  const int lo = t - e * fix_stages(nact, e);
   return lo > 0 ? lo : 0;
 }
-inline int64_t fix_table_entries(int t, int nact) { return (int64_t)1 << (t - fix_table_skip(t, nact)); }
+inline int64_t fix_table_entries(int t, int nact, int e) { return (int64_t)1 << (t - fix_table_skip(t, nact, e)); }
 
 void fix_schedule(FixDesc& d);
-int fix_ctas_per_sm(int t, bool bwd, bool uncompute);
+int fix_ctas_per_sm(const FixDesc& d, bool bwd, bool uncompute);
 cudaError_t launch_fix_tables(const FixTables& ft, const double* params, char* area, cudaStream_t st);
 cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl);
 // chained: history mode, every backward sweep of the call is launched so, and d.early is

@@ -52,9 +52,12 @@ __device__ __forceinline__ void cmul_fix(i64& re, i64& im, int4 d) {
 // with the top ones).  The exchange buffer between stages is XOR-swizzled on
 // 16-byte slots so that the eight lanes of a quarter warp hit eight bank
 // groups in every layout.
-constexpr int E = FIX_E, NA = 1 << E;
+#ifndef QG_FIX_E
+#define QG_FIX_E 3
+#endif
+constexpr int E = QG_FIX_E, NA = 1 << E;
 
-template <int T>
+template <int T, int = QG_FIX_E>  // (a type of its own per translation unit's E)
 struct Lay {
   static constexpr int NT = 1 << (T - E);
   __host__ __device__ static constexpr int sw(int e) { return e ^ ((e >> 3) & 7); }
