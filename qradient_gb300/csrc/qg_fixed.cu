@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
     from_frame<T>(smem, re, im, d, 0);
     store_tile(p.psi_out + x, re, im, s, d.kout[0], d.top);
     // The next launch may come in once every CTA has stored its last tile.
-    // Triggered at the start, as the double kernels do, its CTAs waited on
+    // Triggered at the start, its CTAs waited on
     // the SMs beside this grid's, and filled a few of them when a grid is
     // smaller than the chip holds (n = 18, L = 20: 1.89 -> 1.07 ms).
     if (tile + (int)gridDim.x >= ntiles) pdl_trigger();

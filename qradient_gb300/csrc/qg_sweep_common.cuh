@@ -22,7 +22,7 @@ template <typename R>
 constexpr int kTileFixed = sizeof(R) == 4 ? kTileC64 : kTileC128;
 
 // Programmatic dependent launch.  The sweep and observable kernels let the
-// next launch start at once (pdl_trigger) and, after their setup (which
+// next launch start once their own wait is over (pdl_trigger) and, after their setup (which
 // reads only the angles and the descriptor), wait for the previous grid's
 // completion and memory (pdl_wait) before their first access to a state,
 // the cost tables or the partial sums.  Launched with the attribute after
