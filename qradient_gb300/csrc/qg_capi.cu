@@ -295,12 +295,14 @@ struct FixSweep {
 // Sweeps of one layer: A = bits [0, t), then the high bits, each tile padded
 // with the lowest bits.  A tuned size holds for every tile.  The default,
 // measured per grad_run (ms, L = 20 unless said; t:k per sweep):
-//  - n <= 11: one sweep of one tile (n = 11: 0.60 against 0.63 for 9:9,9:2;
-//    n = 12: 0.94 against 0.66, so two from there on).
+//  - n <= 10: one sweep of one tile (n = 10, L = 10: 0.247 against 0.244 for
+//    8:8,8:2, with half the launches).
 //  - Small states leave SMs idle: the smallest tiles that need two sweeps
-//    (n = 16: 9:9,9:7 0.79, 10:10,10:6 0.83; n = 18: 10:10,10:8 1.07,
-//    9:9,9:9 1.31, 12:12,12:6 1.62; n = 19: 12:12,12:7 1.77, 11:11,11:8
-//    1.91, 10:10,10:9 1.96).
+//    (n = 11, L = 10: 8:8,8:3 0.261, 9:9,9:2 0.262, one tile 0.300; n = 12:
+//    8:8,8:4 0.472, 9:9,9:3 0.498; n = 13: 8:8,8:5 0.493, 9:9,9:4 0.508;
+//    n = 17: 9:9,9:8 0.730, 10:10,10:7 0.761; n = 18, eight amplitudes a
+//    thread: 10:10,10:8 1.07, 9:9,9:9 1.31, 12:12,12:6 1.62; n = 19:
+//    12:12,12:7 1.77, 11:11,11:8 1.91, 10:10,10:9 1.96).
 //  - n = 20, 21 stay in L2, where runs shorter than 128 bytes cost nothing:
 //    two sweeps of 11-bit tiles (n = 20: 2.42; 12:12,12:8 2.62;
 //    10:10,10:5,10:5 2.78).
@@ -330,7 +332,7 @@ std::vector<FixSweep> fix_layout(int n, int tile_bits, bool history) {
     return out;
   }
   if (n <= 21) {
-    const int t = n <= 11 ? n : n <= 16 ? 9 : n <= 18 ? 10 : n == 19 ? 12 : 11;
+    const int t = n <= 10 ? n : n <= 13 ? 8 : n <= 17 ? 9 : n == 18 ? 10 : n == 19 ? 12 : 11;
     out.push_back({t, 0, t});
     if (t < n) rest(t, 1, t);
     return out;
