@@ -696,6 +696,10 @@ __global__ void __launch_bounds__(BfSmem<T>::NT, 512 / BfSmem<T>::NT) batched_fi
         for (int w = 0; w < NW; ++w) q += S.red[w];
         __syncthreads();
         q = over_cluster(q, [](double a, double b) { return a + b; });
+        // lambda with a NaN or an infinity (a non-finite weight, or finite ones
+        // whose sum overflows): fixed point has none to carry on, so the job's
+        // gradient is set to NaN (`big` drops NaN, the squares keep them)
+        if (tid == 0 && !isfinite(q)) S.bad = 1;
         pl = e0 + (q > 0.0 && isfinite(q) ? (ilogb(q) + 2) >> 1 : 0);  // norm^2 < 2^(ilogb + 1)
 #pragma unroll
         for (int c = 0; c < NA; ++c) {
