@@ -343,6 +343,9 @@ __global__ void __launch_bounds__(NT, 1) batched_kernel(const BatchJob* __restri
       __syncthreads();
   };
 
+  // the first job number is written into the other CTAs' shared memory, which
+  // may be touched only once they have started
+  if (CS > 1) cluster.sync();
   for (;;) {
     if (tid == 0 && rank == 0) {
       const int j = atomicAdd(counter, 1);

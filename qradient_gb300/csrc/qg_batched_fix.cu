@@ -162,6 +162,9 @@ __global__ void __launch_bounds__(BfSmem<T>::NT, 512 / BfSmem<T>::NT) batched_fi
       __syncthreads();
   };
 
+  // the first job number is written into the other CTAs' shared memory, which
+  // may be touched only once they have started
+  if (CL) cluster.sync();
   for (;;) {
     if (tid == 0 && rank == 0) {
       const int j = atomicAdd(counter, 1);
