@@ -271,6 +271,12 @@ int qg_batch_workspace_size(size_t* bytes);
 int qg_batch_launch(int dtype, const qg_batch_job* jobs_dev, int njobs, int max_qubits, int cluster,
                     void* workspace_dev, size_t workspace_bytes, qg_stream stream);
 
+/* A stream of the current device that no framework's stream pool hands out
+ * (non-blocking), for callers that launch the groups of a batch side by side.
+ * qg_stream_destroy(NULL) does nothing; work still queued completes. */
+int qg_stream_create(qg_stream* out);
+int qg_stream_destroy(qg_stream stream);
+
 /* ---- Allocation-free gradient (no counterpart in the reference).
  * For callers that cannot allocate device memory where they need a
  * gradient: plug-ins whose host process owns every device allocation

@@ -38,6 +38,8 @@ SIGNATURES = {
                                ctypes.POINTER(_I)]),
     "qg_batch_workspace_size": (_I, [ctypes.POINTER(_SZ)]),
     "qg_batch_launch": (_I, [_I, _P, _I, _I, _I, _P, _SZ, _P]),
+    "qg_stream_create": (_I, [ctypes.POINTER(_P)]),
+    "qg_stream_destroy": (_I, [_P]),
     "qg_grad_noalloc": (_I, [_P, _I, _P, _P, _P, _P, _P]),
     "qg_set_tuning": (_I, [_P, _I, _I, _I, _I]),
     "qg_get_tuning": (_I, [_P, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I)]),

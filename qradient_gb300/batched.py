@@ -14,6 +14,7 @@ depth and observable.
     E, grads = b.grad()                                   # device tensors
 """
 import ctypes
+import weakref
 
 import numpy as np
 import torch
@@ -41,6 +42,48 @@ CLUSTER_MAX = {_lib.QG_C64: 15, _lib.QG_C128: 14}
 MAX_COST = 511
 
 
+class _SideStreams:
+    """Streams for the launch groups of a batch, each held by one Batch at a
+    time.  torch's own streams come round-robin from a pool of 32 per device:
+    taken from there, a group's stream could be one that a server, a graph
+    capture or another thread is using, and the two would wait for each other.
+    Returned streams are kept for the next batch, ``KEEP`` of them at most.
+    (List operations are atomic, and no lock is held when a finalizer runs.)"""
+
+    KEEP = 16
+
+    def __init__(self):
+        self._free = {}  # device index -> stream handles
+
+    def take(self, device, count):
+        lib = _lib.load()
+        index = torch.cuda.current_device() if device.index is None else device.index
+        free = self._free.setdefault(index, [])
+        out = []
+        with torch.cuda.device(index):
+            while len(out) < count:
+                try:
+                    handle = free.pop()
+                except IndexError:
+                    p = ctypes.c_void_p()
+                    _lib.check(lib.qg_stream_create(ctypes.byref(p)))
+                    handle = p.value
+                out.append(torch.cuda.ExternalStream(handle, device=torch.device("cuda", index)))
+            while len(free) > self.KEEP:
+                try:
+                    _lib.check(lib.qg_stream_destroy(free.pop()))
+                except IndexError:
+                    break
+        return out
+
+    def give(self, streams):
+        for st in streams:
+            self._free.setdefault(st.device.index, []).append(st.cuda_stream)
+
+
+_side_streams = _SideStreams()
+
+
 class Batch:
     """A fixed list of jobs executed together; parameters live in ``params``."""
 
@@ -60,6 +103,9 @@ class Batch:
         self._specs = []
         self._graph = None
         self._views = None
+        self._side = []  # this batch's side streams, one per launch group but the first
+        finalizer = weakref.finalize(self, _side_streams.give, self._side)
+        finalizer.atexit = False
         self.finalized = False
 
     # ------------------------------------------------------------ building
@@ -268,6 +314,7 @@ class Batch:
         blob.copy_(torch.from_numpy(host).pin_memory(), non_blocking=True)
         self._blobs = getattr(self, "_blobs", []) + [blob]
         self._big = big
+        self._side += _side_streams.take(dev, len(self._groups) - 1 - len(self._side))
 
     def _structure(self, c, kind):
         """Host-side structure arrays of one circuit (uploaded by the caller)."""
@@ -302,26 +349,28 @@ class Batch:
             _lib.check(lib.qg_batch_launch(self.dtype, _native.ptr(jobs), nj, maxq, cl, _native.ptr(ws), ws.numel(),
                                            _native.stream_handle(self.device)))
 
-        # The groups are independent: all but one go to streams of their own,
+        # The groups are independent: all but one go to the batch's side streams,
         # forked from and joined to the current one, so that a small batch
         # takes as long as its longest job, not the sum over its groups (96
         # complex128 jobs of 8..14 qubits: 6.9 -> 3.9 ms).  Longest jobs first.
         main = torch.cuda.current_stream(self.device)
         groups = self._groups[::-1]
-        side = []
         if len(groups) > 1:
             fork = torch.cuda.Event()
             fork.record(main)
-            for group in groups[1:]:
-                st = torch.cuda.Stream(self.device)
+        forked = []
+        try:
+            for st in self._side[: len(groups) - 1]:
                 st.wait_event(fork)
-                side.append((st, group))
-        for group in groups[:1]:
-            launch(group)
-        for st, group in side:
-            with torch.cuda.stream(st):
-                launch(group)
-            main.wait_stream(st)
+                forked.append(st)
+            if groups:
+                launch(groups[0])
+            for st, group in zip(forked, groups[1:]):
+                with torch.cuda.stream(st):
+                    launch(group)
+        finally:
+            for st in forked:  # also when a launch raised: nothing stays unjoined
+                main.wait_stream(st)
         for i in self._big:
             s = self._specs[i]
             c = s["circuit"]

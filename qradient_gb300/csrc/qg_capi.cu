@@ -1498,4 +1498,17 @@ int qg_batch_launch(int dtype, const qg_batch_job* jobs, int njobs, int max_qubi
   return QG_OK;
 }
 
+int qg_stream_create(qg_stream* out) {
+  if (!out) return fail(QG_ERR_INVALID, "null output");
+  cudaStream_t st = nullptr;
+  QG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  *out = (qg_stream)st;
+  return QG_OK;
+}
+
+int qg_stream_destroy(qg_stream stream) {
+  if (stream) QG_CUDA(cudaStreamDestroy((cudaStream_t)stream));
+  return QG_OK;
+}
+
 }  // extern "C"
