@@ -280,10 +280,18 @@ int build_layer(int n, const Layout& lay, const std::vector<LayerGate>& g, int8_
 // eight amplitudes a thread; n = 8, L = 10: 316 us in the double kernels, 204
 // here), tiles of 8..12 bits, an integer cost, and unless the single-buffered
 // double kernels are asked for.
+// The tile size asked for: a handle's own, else the environment's (5..12, as
+// for the double sweeps), else 0.
+int fixed_tile_setting(const qg_circuit* c) {
+  if (c->tune_tile_bits[0] > 0) return c->tune_tile_bits[0];
+  const int t = env_int("QG_TILE_BITS_C128", 0);
+  return t > 0 ? std::max(5, std::min(t, max_tile_bits(QG_C128))) : 0;
+}
+
 bool fixed_path(const qg_circuit* c, int dtype) {
   if (dtype != QG_C128 || c->n < FIX_TMIN || c->L < 1) return false;
   if (c->kind == 1 && c->cost_kind != COST_INT) return false;
-  const int t = c->tune_tile_bits[0];
+  const int t = fixed_tile_setting(c);
   if (t != 0 && (t < FIX_TMIN || t > FIX_TMAX)) return false;
   return fwd_pipelined(c, dtype);
 }
@@ -377,7 +385,7 @@ int8_t ent_of(const qg_circuit* c) {
 // with every rotation in the sweep that owns its bit.
 void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
   const int n = c->n;
-  const std::vector<FixSweep> lay = fix_layout(n, c->tune_tile_bits[0], op == QG_OP_GRAD_HISTORY);
+  const std::vector<FixSweep> lay = fix_layout(n, fixed_tile_setting(c), op == QG_OP_GRAD_HISTORY);
   const int per = (int)lay.size();
   const bool mc = c->kind == 0;
   const int ini = mc && with_ini ? 1 : 0;
@@ -641,7 +649,10 @@ WsLayout ws_layout(const qg_circuit* c, int dtype, int op, const Program& P) {
     for (const auto& d : P.fix) {
       const int64_t nt = (int64_t)1 << (n - d.t);
       int pf = fix_ctas_per_sm(d, false, unc), pb = fix_ctas_per_sm(d, true, unc);
-      if (tuned > 0) pf = std::min(pf, tuned), pb = std::min(pb, tuned);
+      if (tuned > 0)
+        pf = std::min(pf, tuned), pb = std::min(pb, tuned);
+      else
+        pb = std::max(1, std::min(pb, env_int("QG_CTAS_PER_SM", pb)));
       w.grid_fwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pf));
       w.grid_bwd_k.push_back((int)std::min<int64_t>(nt, (int64_t)sms * pb));
       w.G = std::max(w.G, w.grid_bwd_k.back());
