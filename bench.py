@@ -743,12 +743,13 @@ def main():
         "roofline": roof,
         "clocks": clk,
     }
-    from qradient_gb300 import tuning as _tuning
+    from qradient_gb300 import _native, tuning as _tuning
 
-    t_eff, c_eff, f_eff = _tuning.get_tuning(circ.native(), circ._dtype_code)
-    line["config"]["tile_bits"] = t_eff
-    line["config"]["ctas_per_sm"] = c_eff
-    line["config"]["forward_sweeps"] = "pipelined" if f_eff == _lib.QG_TUNE_FWD_PIPELINED else "plain"
+    plan = _tuning.get_plan(circ.native(), circ._dtype_code,
+                            _native.choose_grad_op(circ.native(), circ._dtype_code, dev, circ.grad_mode))
+    line["config"]["tile_bits"] = [t for t, _ in plan["sweeps"]]
+    line["config"]["ctas_per_sm"] = plan["ctas_per_sm"]
+    line["config"]["sweeps"] = "fixed-point" if plan["fixed_point"] else "floating-point"
     if tuned is not None:
         line["config"]["autotune"] = {"chosen": [tuned["tile_bits"], tuned["ctas_per_sm"], tuned["flags"]],
                                       "ms_by_candidate": {"%d/%d/%d" % (r["tile_bits"], r["ctas_per_sm"], r["flags"]):

@@ -154,16 +154,23 @@ int qg_sample(int n, int dtype, const void* state_dev, int64_t nshots, uint64_t 
  * sweep kernel (0: the default, pipelined).  complex128 sweeps of 8 bits or
  * more run in 64-bit fixed point, which has one forward kernel;
  * QG_TUNE_FWD_PLAIN and tile_bits 5..7 select the double sweeps.
- * qg_get_tuning reports the effective values (tile bits after clamping to n,
- * for a default complex128 handle those of the double sweeps; CTAs per SM of
- * the backward sweeps; the forward kernel flag).  The autotuner of
- * qradient_gb300/tuning.py picks them by timing. */
+ * qg_get_tuning reports these settings as they act on the general (complex64
+ * and double) sweeps: tile bits after clamping to n, CTAs per SM of the
+ * backward sweeps, the forward kernel flag.  qg_get_plan reports the sweeps
+ * that an op runs (with a workspace of qg_workspace_size): whether they are
+ * the fixed-point ones, how many a layer takes, each one's tile bits and the
+ * bits whose rotations it applies (arrays of QG_MAX_QUBITS entries, either may
+ * be NULL), and the resident CTAs per SM of the widest backward grid.  The
+ * autotuner of qradient_gb300/tuning.py picks the settings by timing. */
 enum {
   QG_TUNE_FWD_PIPELINED = 1, /* forward sweeps prefetch the next tile (double-buffered) */
   QG_TUNE_FWD_PLAIN = 2      /* forward sweeps load, compute, store (single buffer) */
 };
 int qg_set_tuning(qg_circuit* c, int dtype, int tile_bits, int ctas_per_sm, int flags);
 int qg_get_tuning(const qg_circuit* c, int dtype, int* tile_bits, int* ctas_per_sm, int* flags);
+enum { QG_MAX_QUBITS = 34 };
+int qg_get_plan(const qg_circuit* c, int dtype, int op, int* fixed_point, int* sweeps_per_layer, int* tile_bits,
+                int* active_bits, int* ctas_per_sm);
 
 /* ---- Finite-shot estimates (the projector estimator of
  * ParametrizedCircuit.sample_expec_val / sample_component_expec_val,

@@ -1414,6 +1414,31 @@ int qg_get_tuning(const qg_circuit* c, int dtype, int* tile_bits, int* ctas_per_
   return QG_OK;
 }
 
+int qg_get_plan(const qg_circuit* c, int dtype, int op, int* fixed_point, int* sweeps_per_layer, int* tile_bits,
+                int* active_bits, int* ctas_per_sm) {
+  static_assert(QG_MAX_QUBITS == QMAX, "one sweep per qubit at most");
+  if (int s = check_circuit(c)) return s;
+  if (dtype != QG_C128 && dtype != QG_C64) return fail(QG_ERR_INVALID, "unknown dtype %d", dtype);
+  if (op < QG_OP_RUN || op > QG_OP_GRAD_UNCOMPUTE) return fail(QG_ERR_INVALID, "unknown op %d", op);
+  if (!fixed_point || !sweeps_per_layer) return fail(QG_ERR_INVALID, "null output");
+  std::shared_ptr<const Plan> plan;
+  if (int s = get_plan(c, dtype, op, false, plan)) return s;
+  const Program& P = plan->P;
+  *fixed_point = P.fixed;
+  *sweeps_per_layer = P.fixed ? P.ft.per_layer : (int)P.lay.tiles.size();
+  for (int k = 0; k < *sweeps_per_layer; ++k) {
+    if (tile_bits) tile_bits[k] = P.fixed ? P.ft.t[k] : (int)P.lay.tiles[k].size();
+    if (active_bits) active_bits[k] = P.fixed ? P.ft.nact[k] : (int)P.lay.active[k].size();
+  }
+  if (ctas_per_sm) {
+    int g = 0;
+    for (int x : plan->W.grid_bwd_k) g = std::max(g, x);
+    const int sms = sm_count();
+    *ctas_per_sm = sms > 0 ? (g + sms - 1) / sms : g;
+  }
+  return QG_OK;
+}
+
 int qg_pauli_workspace_size(const qg_circuit* c, size_t* bytes) {
   if (int s = check_circuit(c)) return s;
   if (!bytes) return fail(QG_ERR_INVALID, "null output");

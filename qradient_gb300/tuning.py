@@ -78,10 +78,22 @@ def set_tuning(native, dtype, tile_bits=0, ctas_per_sm=0, flags=0):
 
 
 def get_tuning(native, dtype):
-    """Effective (tile_bits, ctas_per_sm, flags) of a handle."""
+    """Effective (tile_bits, ctas_per_sm, flags) of a handle, as they act on the
+    general sweeps; ``get_plan`` has the sweeps that run."""
     t, c, f = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     _lib.check(_lib.load().qg_get_tuning(native._h, dtype, ctypes.byref(t), ctypes.byref(c), ctypes.byref(f)))
     return t.value, c.value, f.value
+
+
+def get_plan(native, dtype, op):
+    """The sweeps that `op` (``_lib.QG_OP_*``) runs: {"fixed_point", "sweeps":
+    [(tile bits, active bits) per sweep of a layer], "ctas_per_sm"}."""
+    I = ctypes.c_int
+    fixed, count, ctas, t, k = I(0), I(0), I(0), (I * 34)(), (I * 34)()
+    _lib.check(_lib.load().qg_get_plan(native._h, dtype, op, ctypes.byref(fixed), ctypes.byref(count), t, k,
+                                       ctypes.byref(ctas)))
+    return {"fixed_point": bool(fixed.value), "sweeps": [(t[i], k[i]) for i in range(count.value)],
+            "ctas_per_sm": ctas.value}
 
 
 def sweep_candidates(dtype, n):
