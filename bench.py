@@ -585,6 +585,13 @@ def run_serving(args):
         print(json.dumps(line))
 
 
+def own_launches(steps, profiled, fixed_point):
+    """Kernels of this library in `steps` McClean grad_runs: the profiled ones
+    (sweeps, observable passes), the finaliser and, for the fixed-point
+    sweeps, the phase tables of each."""
+    return profiled + steps * (2 if fixed_point else 1)
+
+
 def backward_profile(dtype, n):
     """ncu's figures of a backward sweep launch of the headline workload
     (profiles/backward_sweep_traffic.json): DRAM bytes and, for complex128,
@@ -730,7 +737,10 @@ def main():
         roof["issue_active_ncu"] = prof.get("issue_active_ncu")
         roof["fp64_pipe_busy_ncu"] = prof.get("fp64_pipe_busy_ncu")
 
-    launches_per_step = (fwd_n + bwd_n + kinfo["observable"][1]) / args.steps + 1  # + the finalize kernel
+    from qradient_gb300 import _native, tuning as _tuning
+
+    plan = _tuning.get_plan(circ.native(), circ._dtype_code,
+                            _native.choose_grad_op(circ.native(), circ._dtype_code, dev, circ.grad_mode))
     line = {
         "metric": "grad_run circuits/s", "value": value, "unit": "circuits/s", "n_gpus": world, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
@@ -739,14 +749,10 @@ def main():
         "hbm_gbs_algorithmic": B * value * 1e-9,
         "e2e": {"value": world / e2e_s, "unit": "circuits/s", "h2d_bytes_per_step": angles.size * 8,
                 "d2h_bytes_per_step": (angles.size + 1) * 8},
-        "gpu_launches": int(round(launches_per_step * args.steps)),
+        "gpu_launches": own_launches(args.steps, fwd_n + bwd_n + kinfo["observable"][1], plan["fixed_point"]),
         "roofline": roof,
         "clocks": clk,
     }
-    from qradient_gb300 import _native, tuning as _tuning
-
-    plan = _tuning.get_plan(circ.native(), circ._dtype_code,
-                            _native.choose_grad_op(circ.native(), circ._dtype_code, dev, circ.grad_mode))
     line["config"]["tile_bits"] = [t for t, _ in plan["sweeps"]]
     line["config"]["ctas_per_sm"] = plan["ctas_per_sm"]
     line["config"]["sweeps"] = "fixed-point" if plan["fixed_point"] else "floating-point"
