@@ -1,6 +1,7 @@
 // Cost tables and the shot sampler.
 #include <stdint.h>
 
+#include "qg_draw.cuh"
 #include "qg_extra.h"
 #include "qg_philox.cuh"
 
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(1024) scan_kernel(const double* sums, int64_t 
 constexpr int DRAW_THREADS = 128, DRAW_SEG = SAMPLE_CHUNK / DRAW_THREADS;
 
 template <typename C>
-__global__ void __launch_bounds__(DRAW_THREADS) draw_kernel(const C* psi, int64_t N, const double* prefix, int64_t nb,
-                                                            int64_t nshots, uint64_t seed, uint64_t offset,
+__global__ void __launch_bounds__(DRAW_THREADS) draw_kernel(const C* psi, int64_t N, const double* sums, const double* prefix,
+                                                            int64_t nb, int64_t nshots, uint64_t seed, uint64_t offset,
                                                             int64_t* out) {
   __shared__ double seg[DRAW_THREADS];      // running sum before each segment
   __shared__ double wtot[DRAW_THREADS / 32];
@@ -141,17 +142,7 @@ __global__ void __launch_bounds__(DRAW_THREADS) draw_kernel(const C* psi, int64_
     uint32_t c[4] = {(uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u};
     philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
     const double u = u01_from(c[0], c[1]) * total;
-    // last chunk with prefix <= u (the same in every thread)
-    int64_t lo = 0, hi = nb - 1;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi + 1) >> 1;
-      if (prefix[mid] <= u)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    // skip empty chunks at the end of the range (rounding)
-    while (lo > 0 && prefix[lo + 1] - prefix[lo] <= 0.0) --lo;
+    const int64_t lo = pick_chunk(prefix, sums, nb, u);  // the same in every thread
     const int64_t x0 = lo * SAMPLE_CHUNK, mine = x0 + tid * DRAW_SEG;
     double sum = 0.0;
     if (mine < N) {
@@ -212,6 +203,7 @@ __global__ void __launch_bounds__(DRAW_THREADS) draw_kernel(const C* psi, int64_
 // n = 8 took 1.65 ms that way (0.41 with a walk per thread, now 0.04), at
 // n = 12 2.7 ms (5.4 and 0.04).
 constexpr int CDF_THREADS = 512, CDF_SEG = SAMPLE_CHUNK / CDF_THREADS;
+static_assert(CDF_SEG == 8, "a byte of weight bits per thread");
 
 template <typename C>
 __global__ void __launch_bounds__(CDF_THREADS) draw_cdf_kernel(const C* psi, int N, const double* prefix,
@@ -219,12 +211,14 @@ __global__ void __launch_bounds__(CDF_THREADS) draw_cdf_kernel(const C* psi, int
                                                                int64_t* out) {
   __shared__ double cdf[SAMPLE_CHUNK];
   __shared__ double wtot[CDF_THREADS / 32];
+  __shared__ uint8_t weight[CDF_THREADS];  // bit i of a byte: its thread's i-th amplitude has weight
   __shared__ int last_nz;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) last_nz = 0;
   double pr[CDF_SEG];
   double sum = 0.0;
   int nz = -1;
+  unsigned bits = 0;
 #pragma unroll
   for (int i = 0; i < CDF_SEG; ++i) {
     const int x = tid * CDF_SEG + i;
@@ -232,7 +226,7 @@ __global__ void __launch_bounds__(CDF_THREADS) draw_cdf_kernel(const C* psi, int
     if (x < N) {
       const C v = psi[x];
       pr[i] = fma((double)v.x, (double)v.x, (double)v.y * (double)v.y);
-      if (pr[i] > 0.0) nz = x;
+      if (pr[i] > 0.0) nz = x, bits |= 1u << i;
     }
     sum += pr[i];
   }
@@ -246,6 +240,7 @@ __global__ void __launch_bounds__(CDF_THREADS) draw_cdf_kernel(const C* psi, int
     run += pr[i];
     cdf[tid * CDF_SEG + i] = run;
   }
+  weight[tid] = (uint8_t)bits;
   if (nz >= 0) atomicMax(&last_nz, nz);
   __syncthreads();
   const double total = prefix[1];
@@ -254,16 +249,7 @@ __global__ void __launch_bounds__(CDF_THREADS) draw_cdf_kernel(const C* psi, int
     uint32_t c[4] = {(uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u};
     philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
     const double u = u01_from(c[0], c[1]) * total;
-    // first index whose running sum exceeds u
-    int lo = 0, hi = N;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (cdf[mid] > u)
-        hi = mid;
-      else
-        lo = mid + 1;
-    }
-    out[s] = lo < N ? lo : last_nz;
+    out[s] = pick_index(cdf, weight, N, u, last_nz);
   }
 }
 
@@ -281,8 +267,8 @@ cudaError_t launch_sample(int n, const C* psi, int64_t nshots, uint64_t seed, ui
     draw_cdf_kernel<C><<<(unsigned)(want < 256 ? want : 256), CDF_THREADS, 0, st>>>(psi, (int)N, prefix, nshots, seed,
                                                                                     offset, out);
   } else if (nshots > 0)
-    draw_kernel<C><<<(unsigned)(nshots < 65536 ? nshots : 65536), DRAW_THREADS, 0, st>>>(psi, N, prefix, nb, nshots,
-                                                                                         seed, offset, out);
+    draw_kernel<C><<<(unsigned)(nshots < 65536 ? nshots : 65536), DRAW_THREADS, 0, st>>>(psi, N, sums, prefix, nb,
+                                                                                         nshots, seed, offset, out);
   return cudaGetLastError();
 }
 
