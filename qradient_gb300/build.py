@@ -30,7 +30,8 @@ def nvcc():
     raise RuntimeError("nvcc not found: the qgrad CUDA library cannot be built")
 
 
-def _deps():
+def sources():
+    """Every file the library is built from."""
     files = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     files.append(os.path.join(INCLUDE, "qgrad.h"))
     return files
@@ -40,7 +41,7 @@ def up_to_date():
     if not os.path.exists(LIB):
         return False
     t = os.path.getmtime(LIB)
-    return all(os.path.getmtime(f) <= t for f in _deps())
+    return all(os.path.getmtime(f) <= t for f in sources())
 
 
 def build(force=False, verbose=False):

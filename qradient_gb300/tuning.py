@@ -16,11 +16,14 @@ distributed shared memory), which halves the shared memory per CTA and the
 per-job latency.  ``tune_batch`` times the batch's graph replay with the
 split starting at different qubit counts and keeps the fastest.
 
-Choices are cached per device, circuit shape and dtype in a JSON file
-(``QG_TUNING_CACHE``, default ``_build/tuning.json`` beside the library), so
-a shape is timed once per machine.
+Choices are cached per device, circuit shape, dtype and gradient mode in a
+JSON file (``QG_TUNING_CACHE``, default ``_build/tuning.json`` beside the
+library), so a shape is timed once per machine.  The keys carry a digest of
+the kernels' sources: a choice timed with other kernels is not applied.
 """
 import ctypes
+import functools
+import hashlib
 import json
 import os
 import threading
@@ -28,7 +31,7 @@ import threading
 import numpy as np
 import torch
 
-from . import _lib, _native
+from . import _lib, _native, build as _build
 
 _LOCK = threading.Lock()
 _MEM = {}
@@ -71,6 +74,17 @@ def _store(key, value):
 
 def _device_tag(device):
     return torch.cuda.get_device_name(device).replace(" ", "_")
+
+
+@functools.lru_cache(maxsize=None)
+def kernel_tag():
+    """Digest of the sources the library is built from."""
+    h = hashlib.sha256()
+    for path in sorted(_build.sources()):
+        h.update(os.path.basename(path).encode())
+        with open(path, "rb") as f:
+            h.update(f.read())
+    return "k" + h.hexdigest()[:12]
 
 
 def set_tuning(native, dtype, tile_bits=0, ctas_per_sm=0, flags=0):
@@ -142,8 +156,8 @@ def _key(circuit, dtype, op, device):
     from .circuit_logic import McClean
 
     kind = "mcclean-%s-%s" % (circuit.entangler, circuit.placement) if isinstance(circuit, McClean) else "qaoa"
-    return "sweep|%s|%s|n%d|%s|%s" % (_device_tag(device), kind, circuit.qnum,
-                                      "c128" if dtype == _lib.QG_C128 else "c64", op)
+    return "sweep|%s|%s|%s|n%d|%s|%s" % (kernel_tag(), _device_tag(device), kind, circuit.qnum,
+                                         "c128" if dtype == _lib.QG_C128 else "c64", op)
 
 
 def tune_circuit(circuit, op="grad", reps=3, layers=4, candidates=None, use_cache=True):
@@ -152,7 +166,11 @@ def tune_circuit(circuit, op="grad", reps=3, layers=4, candidates=None, use_cach
     "timings"}; the timings are per candidate, in ms per call of the copy."""
     dev = circuit._device()
     dtype = circuit._dtype_code
-    key = _key(circuit, dtype, op, dev)
+    # the mode that the circuit itself runs in (the shortened copy's history
+    # would nearly always fit)
+    gop = _native.choose_grad_op(circuit.native(), dtype, dev, getattr(circuit, "grad_mode", "auto"))
+    mode = "" if op != "grad" else "-history" if gop == _lib.QG_OP_GRAD_HISTORY else "-uncompute"
+    key = _key(circuit, dtype, op + mode, dev)
     if use_cache and candidates is None:
         hit = _load().get(key)
         if hit is not None:
@@ -162,7 +180,6 @@ def tune_circuit(circuit, op="grad", reps=3, layers=4, candidates=None, use_cach
     params = torch.rand(max(nparams, 1), dtype=torch.float64, device=dev)[:nparams] * 2 * np.pi
     e = torch.empty(1, dtype=torch.float64, device=dev)
     g = torch.empty(max(nparams, 1), dtype=torch.float64, device=dev)
-    gop = _native.choose_grad_op(nat, dtype, dev, getattr(circuit, "grad_mode", "auto"))
     timings = []
     for t, c, f in candidates or sweep_candidates(dtype, circuit.qnum):
         set_tuning(nat, dtype, t, c, f)
@@ -191,8 +208,8 @@ def tune_batch(batch, reps=3, use_cache=True):
 
     single, cmax = SINGLE_MAX[batch.dtype], CLUSTER_MAX[batch.dtype]
     qs = sorted({s["circuit"].qnum for s in batch._specs})
-    key = "batch|%s|%s|%s" % (_device_tag(batch.device), "c128" if batch.dtype == _lib.QG_C128 else "c64",
-                              ",".join("%d" % q for q in qs))
+    key = "batch|%s|%s|%s|%s" % (kernel_tag(), _device_tag(batch.device),
+                                 "c128" if batch.dtype == _lib.QG_C128 else "c64", ",".join("%d" % q for q in qs))
     choices = [single + 1] + [q for q in range(single, single - 3, -1) if q in qs and q >= 4]
     hit = _load().get(key) if use_cache else None
     if hit is not None and hit["cluster_from"] in choices:
