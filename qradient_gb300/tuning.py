@@ -112,10 +112,12 @@ def get_plan(native, dtype, op):
 
 def sweep_candidates(dtype, n):
     """(tile_bits, ctas_per_sm, flags) triples: the default plan (tile_bits
-    0: the library's per-sweep tile sizes), then three uniform fusion depths
-    around the default, each at the occupancy-sized grid and at 1 CTA per
-    SM, with plain and with pipelined (double-buffered) forward sweeps."""
-    depths = (10, 11, 12) if dtype == _lib.QG_C128 else (11, 12, 13)
+    0: the library's per-sweep tile sizes), then uniform fusion depths around
+    the default (complex128: 8 to 12 bits, from n = 19 on, where 8 and 9 cost
+    a sweep per layer, 10 to 12), each at the occupancy-sized grid and at 1
+    CTA per SM, with plain and with pipelined (double-buffered) forward
+    sweeps."""
+    depths = (11, 12, 13) if dtype == _lib.QG_C64 else (8, 9, 10, 11, 12) if n <= 18 else (10, 11, 12)
     lo = 5 if dtype == _lib.QG_C128 else 6
     depths = sorted({max(lo, min(t, n)) for t in depths})
     return [(0, 0, 0)] + [(t, c, f) for t in depths for c in (0, 1)
