@@ -85,15 +85,6 @@ __device__ __forceinline__ int stage_code(int s, unsigned mx, unsigned my) {
 
 __device__ __forceinline__ int levels_of(int code) { return __popc(code); }
 
-// rounded right shift, and left shift, of a state
-__device__ __forceinline__ void shift_right(i64* re, i64* im, int s) {
-  const i64 h = 1ll << (s - 1);
-#pragma unroll
-  for (int c = 0; c < NA; ++c) {
-    re[c] = (re[c] + h) >> s;
-    im[c] = (im[c] + h) >> s;
-  }
-}
 __device__ __forceinline__ void shift_left(i64* re, i64* im, int s) {
 #pragma unroll
   for (int c = 0; c < NA; ++c) {
@@ -385,13 +376,14 @@ __global__ void __launch_bounds__(BfSmem<T>::NT, 512 / BfSmem<T>::NT) batched_fi
       __syncthreads();  // the next exchange rewrites slots that others read here
     };
 
+    unsigned dither = 0;  // of the step
     // shift so that mm more levels fit
     auto room = [&](int mm, bool both) {
       const int over = h + mm - LIM;
       const int s = over > 0 ? (over + 1) / 2 : 0;
       if (s) {
-        shift_right(pr, pi, s);
-        if (both) shift_right(lr, li, s);
+        shift_right(pr, pi, s, dither);
+        if (both) shift_right(lr, li, s, dither);
         h -= 2 * s;
         sp -= s;
       }
@@ -718,6 +710,7 @@ __global__ void __launch_bounds__(BfSmem<T>::NT, 512 / BfSmem<T>::NT) batched_fi
     for (int step = 0; step <= (grad ? 2 * L : L); ++step) {
       const bool back = step > L, mid = step == L;
       const int i = back ? 2 * L - step : step;
+      dither = dither_bit(rank, step);
       if (!mid) {
         need_units(i, back);
         load_axes(i);

@@ -71,32 +71,28 @@ __device__ __forceinline__ void exchange_at(unsigned char* ex, i64* re, i64* im,
 
 // ------------------------------------------------------------ stages
 
-__device__ __forceinline__ void shift_all(i64* re, i64* im, int s) {
-  if (s == 0) return;
-  const i64 h = 1ll << (s - 1);
-#pragma unroll
-  for (int c = 0; c < NA; ++c) {
-    re[c] = (re[c] + h) >> s;
-    im[c] = (im[c] + h) >> s;
-  }
+__device__ __forceinline__ void shift_all(i64* re, i64* im, int s, unsigned dither) {
+  if (s) shift_right(re, im, s, dither);
 }
 
 // V^-1 on all active bits, from stage 0's layout to the last stage's
 template <int T>
-__device__ __forceinline__ void to_frame(unsigned char* ex, i64* re, i64* im, const FixDesc& d, int dir) {
+__device__ __forceinline__ void to_frame(unsigned char* ex, i64* re, i64* im, const FixDesc& d, int dir,
+                                         unsigned dither) {
 #pragma unroll 1
   for (int s = 0;;) {
     butterflies<true>(re, im, d.code[s]);
     if (++s == opaque(d.nst)) break;
     exchange_at<T, true>(ex, re, im, s);
-    shift_all(re, im, d.sh_in[dir][s]);
+    shift_all(re, im, d.sh_in[dir][s], dither);
   }
 }
 template <int T>
-__device__ __forceinline__ void from_frame(unsigned char* ex, i64* re, i64* im, const FixDesc& d, int dir) {
+__device__ __forceinline__ void from_frame(unsigned char* ex, i64* re, i64* im, const FixDesc& d, int dir,
+                                           unsigned dither) {
 #pragma unroll 1
   for (int s = opaque(d.nst) - 1;;) {
-    shift_all(re, im, d.sh_out[dir][s]);
+    shift_all(re, im, d.sh_out[dir][s], dither);
     butterflies<false>(re, im, d.code[s]);
     if (--s < 0) break;
     exchange_at<T, false>(ex, re, im, s + 1);
@@ -330,6 +326,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const i64 x = tile_base(d, tile) | dep;
     const i64 src = (i64)ladder_inv((uint64_t)x, masks_of(d));
+    const unsigned dither = dither_bit(tile, d.sweep);
     double2 raw[NA];
     if (opaque(d.start) == START_LOAD) {
       load_tile(raw, p.psi_in, opaque(d.pre), x, src, d.top, d.top_inv);
@@ -350,9 +347,9 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
 #pragma unroll
       for (int c = 0; c < NA; ++c) cmul_fix<false>(re[c], im[c], __ldg(ctab + ci[combine(d.top, c)] + d.cost_maxabs));
     }
-    to_frame<T>(smem, re, im, d, 0);
+    to_frame<T>(smem, re, im, d, 0, dither);
     phase_mul<T, false>(re, im, tab, opaque(d.nst));
-    from_frame<T>(smem, re, im, d, 0);
+    from_frame<T>(smem, re, im, d, 0, dither);
     store_tile(p.psi_out + x, re, im, s, d.kout[0], d.top);
     // The next launch may come in once every CTA has stored its last tile.
     // Triggered at the start, its CTAs waited on
@@ -393,6 +390,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const i64 x = tile_base(d, tile) | dep;
     const i64 src = (i64)ladder_fwd((uint64_t)x, masks_of(d));
+    const unsigned dither = dither_bit(tile, d.sweep);
     const bool last = tile + (int)gridDim.x >= ntiles;
     if (EARLY && last && !early) pdl_trigger();
     {
@@ -429,7 +427,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
       }
       const Scale s = tile_scale<T>(raw, N, par, poison);
       load_fix(raw, re, im, s, d.B[1]);
-      to_frame<T>(smem, re, im, d, 1);
+      to_frame<T>(smem, re, im, d, 1, dither);
       if (st == 0) {
 #pragma unroll
         for (int c = 0; c < NA; ++c) park[c * NT + tid] = make_longlong2(re[c], im[c]);
@@ -477,7 +475,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
         }
       }
       phase_mul<T, true>(re, im, tab, opaque(d.nst));
-      from_frame<T>(smem, re, im, d, 1);
+      from_frame<T>(smem, re, im, d, 1, dither);
       if (opaque(d.cost) == COST_INT) {
         const int32_t* ci = p.cost_i + x;
 #pragma unroll
