@@ -236,22 +236,27 @@ __device__ __forceinline__ Scale tile_scale(double2* v, NormShared<T>& N, int& p
   return r;
 }
 
-// floor(x * 2^k) in integer instructions: half of the conversions take this
-// form, so that the FP64 pipe (16 cycles per conversion) and the integer
-// pipes share them (n = 24, L = 20: 28.9 ms; all in this form 29.9, none 31).  (Floor, not truncation: an error that follows the sign
-// would shrink the norm a little in every sweep.)
-__device__ __forceinline__ i64 to_fix_int(double x, int k) {
+// x * 2^k to the nearest integer in integer instructions, |x * 2^k| < 2^62:
+// half of the conversions take this form, so that the FP64 pipe (16 cycles per
+// conversion) and the integer pipes share them (a half, a quarter, none: n = 20,
+// L = 50 5.82, 6.05, 6.22 ms; n = 24 72.7, 72.0, 74.0).  `tie` 2 rounds ties
+// up, 0 down, whatever the sign (see dither_bit).  Rounded down instead, as
+// this was (n = 24 70.3 ms), every imaginary part was half a unit low, the
+// same way in every sweep: gradients by small X angles 1.1e-13 off at n = 14
+// and 20 layers (now 2.3e-15, double sweeps 2.2e-15), QAOA with small angles
+// 2.1e-14 at n = 16 (2e-16, 4.0e-15).  All ties up: 9e-15 and 2.3e-15.
+__device__ __forceinline__ i64 to_fix_int(double x, int k, unsigned tie) {
   const int hi = __double2hiint(x), sg = hi >> 31;
-  // negative values in ones' complement (its distance to the two's complement
-  // lies below the rounding); leading one at bit 62: value 2^(ex - 1085)
+  // leading one at bit 61: |value| 2^(ex - 1084); negative values in ones'
+  // complement, one less than the two's: `tie` - 1 beside it is 1 or -1
   const unsigned l = (unsigned)(__double2loint(x) ^ sg), h = (unsigned)(hi ^ sg);
-  const unsigned top = ((unsigned)sg & 0xc0000000u) ^ 0x40000000u;
-  const unsigned mh = (__funnelshift_l(l, h, 10) & 0x3fffffffu) | top;
-  const int r = 1085 - k - ((hi >> 20) & 0x7ff);
-  const i64 m = (i64)((uint64_t)mh << 32 | __funnelshift_l((unsigned)sg, l, 10));
-  i64 d;
-  asm("shr.s64 %0, %1, %2;" : "=l"(d) : "l"(m), "r"(r));  // (clamps r > 63)
-  return d;
+  const unsigned top = ((unsigned)sg & 0xe0000000u) ^ 0x20000000u;
+  const unsigned mh = (__funnelshift_l(l, h, 9) & 0x1fffffffu) | top;
+  const int r = min(1084 - k - ((hi >> 20) & 0x7ff), 63);  // 0..63 (beyond: below a quarter, as at 63)
+  const i64 m = (i64)((uint64_t)mh << 32 | __funnelshift_l((unsigned)sg, l, 9));
+  uint64_t below;  // 2^(r-1) - 1, or 0 for r < 2: a whole number then, off by two of 2^60 at most
+  asm("shr.u64 %0, %1, %2;" : "=l"(below) : "l"(~0ull), "r"(65 - r));
+  return (m + (i64)below + (i64)(uint64_t)tie) >> r;
 }
 // x * 2^k to the nearest integer; |x * 2^k| < 2^63
 __device__ __forceinline__ i64 to_fix(double x, int k) {
@@ -265,12 +270,13 @@ __device__ __forceinline__ double from_fix(i64 X, int k) {
   const int hi = __double2hiint(v);
   return __hiloint2double(hi ? hi - (k << 20) : 0, __double2loint(v));
 }
-__device__ __forceinline__ void load_fix(const double2* raw, i64* re, i64* im, const Scale& s, int B) {
+__device__ __forceinline__ void load_fix(const double2* raw, i64* re, i64* im, const Scale& s, int B, unsigned dither) {
   const int k = B - s.p;
+  const unsigned a = 2 * dither, b = 2 - a;
 #pragma unroll
   for (int c = 0; c < NA; ++c) {
     re[c] = to_fix(raw[c].x, k);
-    im[c] = to_fix_int(raw[c].y, k);
+    im[c] = to_fix_int(raw[c].y, k, dither_odd(c) ? a : b);
   }
 }
 
@@ -341,7 +347,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
     }
     const Scale s = tile_scale<T>(raw, N, par, poison);
     i64 re[NA], im[NA];
-    load_fix(raw, re, im, s, d.B[0]);
+    load_fix(raw, re, im, s, d.B[0], dither);
     if (opaque(d.cost) == COST_INT) {
       const int32_t* ci = p.cost_i + x;
 #pragma unroll
@@ -426,7 +432,7 @@ __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 
         }
       }
       const Scale s = tile_scale<T>(raw, N, par, poison);
-      load_fix(raw, re, im, s, d.B[1]);
+      load_fix(raw, re, im, s, d.B[1], dither);
       to_frame<T>(smem, re, im, d, 1, dither);
       if (st == 0) {
 #pragma unroll

@@ -1,8 +1,8 @@
 """complex128 results against the oracle in extended precision, beside those of
 the double sweeps: random circuits, and ones whose amplitudes are alike (small
 angles, one axis, one angle per layer, uniform states), where a rounding that
-always goes one way adds up instead of averaging out.  The batched kernel in
-one CTA and on clusters.
+always goes one way adds up instead of averaging out.  The sweeps in history
+and uncompute form and the batched kernel in one CTA and on clusters.
 
 The measure is the rms over a few circuits of the gradient error's norm.  Two
 terms bound it:
@@ -17,7 +17,8 @@ terms bound it:
   |lambda| 2^-57 2^(-(n-t)/2) 0.29 sqrt(4 * 4 m) over the m sweeps of the
   circuit, forward and backward (batched kernel: t = n).
 
-(Right shifts that rounded every tie up were up to twenty times further off.)"""
+(Rounding imaginary parts down on load, and ties up in the right shifts, was
+up to a hundred times further off.)"""
 import numpy as np
 import pytest
 
@@ -106,4 +107,24 @@ def test_batched_gradient_error(case):
             batch = Batch(dtype="complex128", use_graph=False, cluster_from=first)
             batch.add(c, params=(b if kind == "mc" else np.stack([a, b], 1)).reshape(-1))
             errors.note("batch from %d" % first, batch.grad()[1][0].cpu().numpy(), g0, _step(lam, n, n, L))
+    errors.check()
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c[:5])))
+def test_sweep_gradient_error(case):
+    from qradient_gb300 import _lib, tuning
+
+    n, L, count = case[1], case[2], case[5]
+    errors = _Errors()
+    for seed in range(count):
+        a, b, t = _inputs(case, seed)
+        g0, lam = _exact(case, a, b, t)
+        for name, mode, op, flags in (("double", "history", _lib.QG_OP_GRAD_HISTORY, _lib.QG_TUNE_FWD_PLAIN),
+                                      ("history", "history", _lib.QG_OP_GRAD_HISTORY, 0),
+                                      ("uncompute", "uncompute", _lib.QG_OP_GRAD_UNCOMPUTE, 0)):
+            c, args = _circuit(case, a, b, t, mode, flags)
+            plan = tuning.get_plan(c.native(), c._dtype_code, op)
+            assert plan["fixed_point"] == (name != "double")
+            errors.note(name, c.grad_run(*args)[1], g0,
+                        _step(lam, n, max(t for t, _ in plan["sweeps"]), L * len(plan["sweeps"])))
     errors.check()
