@@ -24,7 +24,7 @@
 #include "../../include/qgrad.h"
 #include "qg_batched.h"
 #include "qg_extra.h"
-#include "qg_fixed.h"
+#include "qg_fixed_layout.cuh"
 #include "qg_internal.cuh"
 #include "qg_kernels.h"
 #include "qg_ladder.cuh"

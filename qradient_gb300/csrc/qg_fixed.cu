@@ -14,14 +14,17 @@
 // one w_x = Im(conj(lam_x) psi_x) per amplitude for all qubits.
 //
 // Number format.  States stay complex128 in memory.  A tile is loaded, scaled
-// by a power of two that puts its 2-norm just below 2^B (B = 60..62), and
-// rounded to int64; sums are exact; products keep the top 64 of 128 bits.
+// by a power of two that puts its 2-norm below 2^B (B = 58..62), and rounded to
+// int64; sums are exact; products keep the top 64 of 128 bits.
 // The norm bounds every component at every later point, because V, D are
 // unitary up to the known factor sqrt(2) per butterfly level, so right shifts
 // scheduled from the level counts alone (fix_schedule) rule out overflow.
-// With 2^12 components the typical one is 2^53.5 units at 2^60: the rounding
-// of a whole sweep (one conversion, at most four shifts, one product) is
-// below that of the double rotations it replaces.
+// A unit is at most 2^-57 of the tile's norm.  The typical one of 2^12
+// components keeps 52 bits or more; the rounding of a whole sweep (one
+// conversion, at most four shifts, one product) is below that of the double
+// rotations it replaces.  Components far below the tile's norm keep fewer bits
+// (relative to themselves) than double would: results are as close as the
+// double sweeps' in norm, not element by element.
 //
 // Reference mapping (qradient, pure numpy):
 //   rotations          physical_components/state.py:90-97, 142-149, 168-175
@@ -730,52 +733,6 @@ cudaError_t FIXFN(launch_fix_bwd)(const FixDesc& d, const FixPtrs& p, bool uncom
 }
 
 #if QG_FIX_E == 3
-// The scaling of a sweep, from the number of its butterfly levels alone.  h
-// counts half bits of the tile's norm above 2^60: a level adds one, a phase
-// product takes eight (its table is scaled by 2^60), the cost product four
-// (2^62), a shift by s takes 2 s.  LIM = 5 keeps the norm, and so every
-// component and every sum inside a product, below 2^62.5.  Up to nine levels
-// need no shift: the tile is loaded at the B (58..62) that lets V^-1 grow to
-// LIM, and the phase product makes the room that V needs.
-void fix_schedule(FixDesc& d) {
-  constexpr int LIM = 5;
-  int m[FIX_STAGES] = {};
-  int levels = 0;
-  for (int s = 0; s < d.nst; ++s) {
-    for (int i = 0; i < FIX_E; ++i) m[s] += ((d.code[s] >> (2 * i)) & 3) != 0;
-    levels += m[s];
-  }
-  for (int dir = 0; dir < 2; ++dir) {
-    int total = 0;  // right shifts so far
-    int h;
-    if (dir == 0 && d.cost == COST_INT) {
-      d.B[0] = 62;
-      h = 0;  // after the cost product
-      total += 2;
-    } else {
-      const int up = levels <= LIM ? (LIM - levels) / 2 : -((levels - LIM + 1) / 2);
-      d.B[dir] = (int8_t)(60 + std::max(-2, std::min(2, up)));
-      h = 2 * (d.B[dir] - 60);
-    }
-    auto room = [&](int mm) {
-      const int over = h + mm - LIM;
-      const int s = over > 0 ? (over + 1) / 2 : 0;
-      h += mm - 2 * s;
-      total += s;
-      return (int8_t)s;
-    };
-    d.sh_in[dir][0] = 0;
-    h += m[0];
-    for (int s = 1; s < d.nst; ++s) d.sh_in[dir][s] = room(m[s]);
-    if (dir == 1) d.kw = (int16_t)(64 - 2 * d.B[1] - levels + 2 * total);
-    h -= 8;
-    total += 4;
-    for (int s = d.nst - 1; s >= 0; --s) d.sh_out[dir][s] = room(m[s]);
-    if (dir == 1 && d.cost == COST_INT) total += 2;
-    d.kout[dir] = (int16_t)(-d.B[dir] - levels + total);
-  }
-}
-
 cudaError_t launch_fix_tables(const FixTables& f, const double* params, char* area, cudaStream_t st) {
   const int grid = f.nsweeps < 1 ? 1 : f.nsweeps < 1024 ? f.nsweeps : 1024;
   fix_tables_kernel<<<grid, 256, 0, st>>>(f, params, area);

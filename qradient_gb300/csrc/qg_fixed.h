@@ -82,7 +82,6 @@ __host__ __device__ inline int fix_table_skip(int t, int nact, int e) {
 }
 inline int64_t fix_table_entries(int t, int nact, int e) { return (int64_t)1 << (t - fix_table_skip(t, nact, e)); }
 
-void fix_schedule(FixDesc& d);
 int fix_ctas_per_sm(const FixDesc& d, bool bwd, bool uncompute);
 cudaError_t launch_fix_tables(const FixTables& ft, const double* params, char* area, cudaStream_t st);
 cudaError_t launch_fix_fwd(const FixDesc& d, const FixPtrs& p, int grid, cudaStream_t st, bool pdl);

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "qg_fixed.h"
+#include "qg_fixed_layout.cuh"
 
 namespace qg {
 
@@ -44,38 +45,6 @@ __device__ __forceinline__ void cmul_fix(i64& re, i64& im, int4 d) {
   re = mad_wide(i.h, -sh, mad_wide(r.h, d.x, m >> 32));
   im = mad_wide(r.h, sh, mad_wide(i.h, d.x, q >> 32));
 }
-
-// ------------------------------------------------------------ layouts
-//
-// A thread holds NA = 2^E amplitudes; stage s has local bits T-E(s+1)..T-Es-1
-// in the thread (the last stage, where fewer remain, the r low bits filled up
-// with the top ones).  The exchange buffer between stages is XOR-swizzled on
-// 16-byte slots so that the eight lanes of a quarter warp hit eight bank
-// groups in every layout.
-#ifndef QG_FIX_E
-#define QG_FIX_E 3
-#endif
-constexpr int E = QG_FIX_E, NA = 1 << E;
-
-template <int T, int = QG_FIX_E>  // (a type of its own per translation unit's E)
-struct Lay {
-  static constexpr int NT = 1 << (T - E);
-  __host__ __device__ static constexpr int sw(int e) { return e ^ ((e >> 3) & 7); }
-  // local index of (thread 0, in-thread index c)
-  __host__ __device__ static constexpr int eoff(int s, int c) {
-    const int lo = T - E * (s + 1);
-    if (lo >= 0) return c << lo;
-    const int r = E + lo;  // low bits in the thread
-    return (c & ((1 << r) - 1)) | ((c >> r) << (T + lo));
-  }
-  // local index of (thread tid, in-thread index 0)
-  __host__ __device__ static constexpr int ebase(int s, int tid) {
-    const int lo = T - E * (s + 1);
-    if (lo >= 0) return (tid & ((1 << lo) - 1)) | ((tid >> lo) << (lo + E));
-    return tid << (E + lo);
-  }
-  static constexpr int NS = (T + E - 1) / E;
-};
 
 // V^-1 (INV) or V on the in-thread bits of a stage, times sqrt(2) per X/Y bit:
 //   X: V^-1 = [[1, 1], [-1, 1]], V = [[1, -1], [1, 1]]
