@@ -103,6 +103,15 @@ int qg_num_params(const qg_circuit* c, int* nparams);
 /* Device workspace bytes for an operation (qg_op) at a dtype. */
 int qg_workspace_size(const qg_circuit* c, int dtype, int op, size_t* bytes);
 
+/* Accuracy in complex128.  From n = 8 on the sweeps, and the batched kernel at
+ * any n, work in 64-bit fixed point under one exponent per tile of 2^8..2^12
+ * amplitudes (batched: per state).  Results are accurate in norm: a sweep adds
+ * an error of at most a few 2^-57 of the tile's norm to an amplitude, whatever
+ * that amplitude's own size.  So an amplitude 10^-17 of its tile's norm is
+ * rounding noise, where double arithmetic would have kept its leading digits
+ * in circuits that hardly mix it with larger ones (angles near 0).  A handle
+ * set to QG_TUNE_FWD_PLAIN (qg_set_tuning) runs the double sweeps. */
+
 /* Forward run and exact expectation value <psi|O|psi> (run_expec_val with
  * exact_expec_val=True).  params_dev: double [nparams].  ini_state_dev:
  * optional start state (NULL: |0..0> for McClean, |+..+> for QAOA); McClean
