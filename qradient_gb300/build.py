@@ -32,7 +32,7 @@ def nvcc():
 
 def sources():
     """Every file the library is built from."""
-    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    files = [f for f in (os.path.join(CSRC, name) for name in os.listdir(CSRC)) if os.path.isfile(f)]
     files.append(os.path.join(INCLUDE, "qgrad.h"))
     return files
 
