@@ -242,7 +242,7 @@ __device__ __forceinline__ Scale tile_scale(double2* v, NormShared<T>& N, int& p
 // x * 2^k to the nearest integer in integer instructions, |x * 2^k| < 2^62:
 // half of the conversions take this form, so that the FP64 pipe (16 cycles per
 // conversion) and the integer pipes share them (a half, a quarter, none: n = 20,
-// L = 50 5.82, 6.05, 6.22 ms; n = 24 72.7, 72.0, 74.0).  `tie` 2 rounds ties
+// L = 50 5.80, 6.05, 6.22 ms; n = 24 72.1, 72.0, 74.0).  `tie` 2 rounds ties
 // up, 0 down, whatever the sign (see dither_bit).  Rounded down instead, as
 // this was (n = 24 70.3 ms), every imaginary part was half a unit low, the
 // same way in every sweep: gradients by small X angles 1.1e-13 off at n = 14
@@ -250,13 +250,12 @@ __device__ __forceinline__ Scale tile_scale(double2* v, NormShared<T>& N, int& p
 // 2.1e-14 at n = 16 (2e-16, 4.0e-15).  All ties up: 9e-15 and 2.3e-15.
 __device__ __forceinline__ i64 to_fix_int(double x, int k, unsigned tie) {
   const int hi = __double2hiint(x), sg = hi >> 31;
-  // leading one at bit 61: |value| 2^(ex - 1084); negative values in ones'
+  // leading one at bit 61: |value| = m 2^(ex - 1084); negative values in ones'
   // complement, one less than the two's: `tie` - 1 beside it is 1 or -1
-  const unsigned l = (unsigned)(__double2loint(x) ^ sg), h = (unsigned)(hi ^ sg);
-  const unsigned top = ((unsigned)sg & 0xe0000000u) ^ 0x20000000u;
-  const unsigned mh = (__funnelshift_l(l, h, 9) & 0x1fffffffu) | top;
+  const unsigned lo = (unsigned)__double2loint(x);
+  const unsigned mh = ((__funnelshift_l(lo, (unsigned)hi, 9) & 0x1fffffffu) | 0x20000000u) ^ (unsigned)sg;
   const int r = min(1084 - k - ((hi >> 20) & 0x7ff), 63);  // 0..63 (beyond: below a quarter, as at 63)
-  const i64 m = (i64)((uint64_t)mh << 32 | __funnelshift_l((unsigned)sg, l, 9));
+  const i64 m = (i64)((uint64_t)mh << 32 | ((lo << 9) ^ (unsigned)sg));
   uint64_t below;  // 2^(r-1) - 1, or 0 for r < 2: a whole number then, off by two of 2^60 at most
   asm("shr.u64 %0, %1, %2;" : "=l"(below) : "l"(~0ull), "r"(65 - r));
   return (m + (i64)below + (i64)(uint64_t)tie) >> r;
@@ -264,7 +263,7 @@ __device__ __forceinline__ i64 to_fix_int(double x, int k, unsigned tie) {
 // x * 2^k to the nearest integer; |x * 2^k| < 2^63
 __device__ __forceinline__ i64 to_fix(double x, int k) {
   // the exponent field moves by k; zeros and denormals become a value below
-  // one half for every k < 1022, and 9 <= k <= 92 on this path
+  // one half for every k < 1022, and 7 <= k <= 91 on this path
   return __double2ll_rn(__hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x)));
 }
 // X * 2^-k
