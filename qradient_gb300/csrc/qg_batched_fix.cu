@@ -5,10 +5,11 @@
 // backward, 16 cycles of the pipe each per warp.  Here a layer of rotations
 // is V D V^-1 as in the fixed-point sweeps (qg_fixed.cu): additions, one
 // phase product, additions; and all gradient sums of a layer come from one
-// product per amplitude.  Psi and lambda stay in registers, eight amplitudes
-// of each per thread, for the whole circuit; shared memory only carries the
-// exchanges between layouts, the CNOT ladder's gather and (across a cluster)
-// the split bits.
+// product per amplitude.  Psi and lambda stay with their threads, eight
+// amplitudes of each, for the whole circuit: in registers, of which the
+// compiler spills 1.4-1.5 KB a thread (480-byte frame) at the cap of 128.
+// Shared memory only carries the exchanges between layouts, the
+// CNOT ladder's gather and (across a cluster) the split bits.
 //
 // Number format.  Rotations keep ||psi|| = 1 and ||lambda||, so one power of
 // two per state scales it to int64 from start to end: no conversion per
@@ -16,11 +17,11 @@
 // butterfly level adds one, the phase product (phases at 2^62) takes four,
 // shifts keep h <= 5 and bring it back to at least 1 before a phase product.
 //
-// Measured (GB300, L = 30, circuits/s, double form -> this): n = 10 114k ->
-// 417k, n = 11 74k -> 280k, n = 12 41k -> 132k, n = 13 (2 CTAs) 18.4k ->
-// 48.5k, n = 14 (4 CTAs) 7.8k -> 18.0k; one n = 12 job alone 3.57 -> 1.09 ms.
-// What bounds it now is instruction issue (44% active at the one CTA of 16
-// warps that 176 KB of shared memory leave room for).
+// Measured (GB300, L = 30, circuits/s, double form -> this, batches of 4096 to
+// 1024 jobs): n = 10 114k -> 476k, n = 11 74k -> 269k, n = 12 41k -> 131k,
+// n = 13 (2 CTAs) 18.4k -> 48.5k, n = 14 (4 CTAs) 7.8k -> 18.3k; one n = 12 job
+// alone 3.57 -> 1.14 ms.  What bounds it now is instruction issue (45% active
+// at the one CTA of 16 warps that 184 KB of shared memory leave room for).
 #include <cooperative_groups.h>
 #include <stdint.h>
 

@@ -277,7 +277,7 @@ int build_layer(int n, const Layout& lay, const std::vector<LayerGate>& g, int8_
 
 // complex128 circuits run on the fixed-point sweeps wherever those have an
 // instantiation: from 8 qubits on (a tile of fewer is less than a warp of
-// eight amplitudes a thread; n = 8, L = 10: 316 us in the double kernels, 204
+// eight amplitudes a thread; n = 8, L = 10: 276 us in the double kernels, 140
 // here), tiles of 8..12 bits, an integer cost, and unless the single-buffered
 // double kernels are asked for.
 // The tile size asked for: a handle's own, else the environment's (5..12, as
@@ -302,23 +302,23 @@ struct FixSweep {
 
 // Sweeps of one layer: A = bits [0, t), then the high bits, each tile padded
 // with the lowest bits.  A tuned size holds for every tile.  The default,
-// measured per grad_run (ms, L = 20 unless said; t:k per sweep):
-//  - n <= 10: one sweep of one tile (n = 10, L = 10: 0.247 against 0.244 for
-//    8:8,8:2, with half the launches).
+// measured per grad_run on the device (ms, L = 20 unless said; t:k per sweep):
+//  - n <= 10: one sweep of one tile (n = 10, L = 10: 0.217; 8:8,8:2 with eight
+//    amplitudes a thread 0.282, with four 0.206 but twice the launches).
 //  - Small states leave SMs idle: the smallest tiles that need two sweeps
-//    (n = 11, L = 10: 8:8,8:3 0.261, 9:9,9:2 0.262, one tile 0.300; n = 12:
-//    8:8,8:4 0.472, 9:9,9:3 0.498; n = 13: 8:8,8:5 0.493, 9:9,9:4 0.508;
-//    n = 17: 9:9,9:8 0.730, 10:10,10:7 0.761; n = 18, eight amplitudes a
-//    thread: 10:10,10:8 1.07, 9:9,9:9 1.31, 12:12,12:6 1.62; n = 19:
-//    12:12,12:7 1.77, 11:11,11:8 1.91, 10:10,10:9 1.96).
+//    (n = 11, L = 10: 8:8,8:3 0.225, 9:9,9:2 0.229, one tile 0.268; n = 12:
+//    8:8,8:4 0.438, 9:9,9:3 0.465, 10:10,10:2 0.545; n = 13: 8:8,8:5 0.459,
+//    9:9,9:4 0.488; n = 17: 9:9,9:8 0.710, 10:10,10:7 0.744; n = 18, eight
+//    amplitudes a thread: 10:10,10:8 0.956, 9:9,9:9 1.18, 12:12,12:6 1.41;
+//    n = 19: 12:12,12:7 1.63, 11:11,11:8 1.69, 10:10,10:9 1.75).
 //  - n = 20, 21 stay in L2, where runs shorter than 128 bytes cost nothing:
-//    two sweeps of 11-bit tiles (n = 20: 2.42; 12:12,12:8 2.62;
-//    10:10,10:5,10:5 2.78).
+//    two sweeps of 11-bit tiles (n = 20: 2.23; 12:12,12:8 2.45;
+//    10:10,10:7,10:3 2.65; n = 21: 4.05, 12:12,12:9 4.32).
 //  - From 22 on three sweeps (four from 31), 128-byte runs, and 10-bit tiles
-//    where they suffice (n = 24, L = 10: 14.3; 11:11,11:8,11:5 15.6;
-//    9:9,9:6,9:6,9:3 14.9).  From n = 28 four sweeps of 10-bit tiles are
+//    where they suffice (n = 24, L = 10: 14.6; 11:11,11:8,11:5 15.1;
+//    9:9,9:6,9:6,9:3 16.0).  From n = 28 four sweeps of 10-bit tiles are
 //    faster than three of 11- and 12-bit ones (n = 28, L = 2 uncompute:
-//    65.7; 12:12,11:8,11:8 70.4), but a history would hold a third more
+//    65.6; 12:12,11:8,11:8 68.1), but a history would hold a third more
 //    states, so that form keeps three.
 std::vector<FixSweep> fix_layout(int n, int tile_bits, bool history) {
   std::vector<FixSweep> out;
@@ -394,10 +394,11 @@ void build_fixed(const qg_circuit* c, int op, bool with_ini, Program& P) {
   memset(&f, 0, sizeof f);
   // Amplitudes a thread.  Up to 17 qubits an SM has one or two tiles and a
   // sweep lasts as long as a warp's own instructions: with four, half of them
-  // (n = 12, L = 20: 603 -> 489 us; n = 15: 662 -> 546; n = 17: 817 -> 763;
-  // n = 18, with more warps than the chip can issue for, 976 -> 1307).  One
-  // tile of 10 or 11 bits has the warps already, and fewer stages with eight
-  // (n = 10, L = 10: 237 against 247 us; n = 11: 309 against 415).
+  // (n = 8, L = 10: 182 -> 138 us; n = 12, L = 20: 603 -> 438; n = 15: 640 ->
+  // 529; n = 17: 766 -> 710; n = 18, with more warps than the chip can issue
+  // for, 956 -> 1292).  One tile of 11 bits has the warps already, and fewer
+  // stages with eight; one of 10 is near even (n = 10, L = 10: 217 us with
+  // eight, 206 with four).
   f.e = n <= 17 && (per > 1 || n < 10) ? 2 : FIX_E;
   for (const FixSweep& s : lay)
     if (s.t > FIX_TMAX2) f.e = FIX_E;
@@ -1027,9 +1028,9 @@ int do_grad(const qg_circuit* c, int op, const double* params, const void* ini, 
   C* psi0 = (C*)(ws + W.psi);
   const int m = P.nsweeps();
   // Overlap neighbouring sweeps (fix_bwd_kernel) where a CTA has at most four
-  // tiles: n = 21, L = 10 2.27 -> 2.10 ms; with more the overlap is a small
+  // tiles: n = 21, L = 10 2.28 -> 2.08 ms; with more the overlap is a small
   // part and the kernel with the wait at its head is the faster one (n = 24,
-  // L = 10: 14.43 against 14.54 ms; n = 22 the same).
+  // L = 10: 14.60 against 14.65 ms; n = 22 3.91 against 3.88).
   bool chained = history && P.fixed;
   for (int k = P.first_param; chained && k < m; ++k)
     chained = ((int64_t)1 << (c->n - P.fix[k].t)) <= 4 * (int64_t)W.grid_bwd_k[k];

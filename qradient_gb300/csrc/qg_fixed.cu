@@ -305,7 +305,7 @@ __device__ __forceinline__ void store_tile(double2* out, const i64* re, const i6
 
 // Prefetch into L2 the 128-byte lines of a tile, one of eight amplitudes per
 // thread, or two threads to a line (their images under the ladder share a line as well).  Backward
-// only: 309 -> 302 us per sweep at n = 24; the forward sweeps lost 3%.
+// only: n = 24, L = 20 28.98 -> 28.83 ms; the forward sweeps lost 3%.
 template <int T>
 __device__ __forceinline__ i64 line_index(const FixDesc& d) {
   const int t = threadIdx.x << E;
@@ -316,7 +316,10 @@ __device__ __forceinline__ void prefetch_line(const double2* p) { asm volatile("
 // ------------------------------------------------------------ forward
 
 // Resident warps per SM that the registers are capped for (64 and 80 a
-// thread): with 24 and 16, n = 24, L = 20 took 29.6 against 28.9 ms.
+// thread).  At these caps the sweeps of up to 11 bits spill 56-204 bytes a
+// thread; with 24 and 16 warps (80 and 128 registers) nothing spills, and
+// n = 24, L = 20 takes 29.6 against 28.8 ms (n = 22, L = 10 3.82 against 3.92,
+// n = 18, L = 20 933 against 965 us).
 constexpr int fwd_warps = 32, bwd_warps = 24;
 
 template <int T>
@@ -374,9 +377,9 @@ __global__ void __launch_bounds__(Lay<T>::NT, fwd_warps / (Lay<T>::NT / 32))
 // into the frame before it waits for the sweep ahead of it, which lets it in
 // as it starts on its last tile (after its own wait, so that the chain is two
 // deep and everything up to the sweep before the last is complete).  n = 10,
-// L = 10: 269 -> 246 us; n = 15, L = 20: 753 -> 677; n = 17: 904 -> 824;
-// n = 18: 1068 -> 985; n = 20: 2429 -> 2265.  Triggered before the wait,
-// waiting CTAs piled up on some SMs (n = 18: 1498).
+// L = 10: 248 -> 223 us; n = 15, L = 20: 590 -> 525; n = 17: 759 -> 706;
+// n = 18: 1057 -> 965; n = 20: 2400 -> 2233.  Triggered before the wait,
+// waiting CTAs piled up on some SMs (n = 18: 985 -> 1498).
 template <int T, bool UNCOMPUTE, bool EARLY>
 __global__ void __launch_bounds__(Lay<T>::NT, bwd_warps / (Lay<T>::NT / 32) > 0 ? bwd_warps / (Lay<T>::NT / 32) : 1)
     fix_bwd_kernel(const __grid_constant__ FixDesc d, FixPtrs p) {
