@@ -1,17 +1,29 @@
 """bench.py's count of the library's own kernels in a grad_run against the
-profiler's list of what was launched."""
+kernel nodes of the call captured in a CUDA graph."""
+import ctypes
+
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,dtype", [(9, "complex128"), (13, "complex128"), (6, "complex128"), (13, "complex64")])
-def test_count_matches_the_profiler(n, dtype):
-    import ctypes
+def _kernel_nodes(graph):
+    drv, P = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p
+    count = ctypes.c_size_t()
+    assert drv.cuGraphGetNodes(P(graph), None, ctypes.byref(count)) == 0
+    nodes = (P * count.value)()
+    assert drv.cuGraphGetNodes(P(graph), nodes, ctypes.byref(count)) == 0
+    kernels, kind = 0, ctypes.c_int()
+    for node in nodes:
+        assert drv.cuGraphNodeGetType(P(node), ctypes.byref(kind)) == 0
+        kernels += kind.value == 0  # CU_GRAPH_NODE_TYPE_KERNEL
+    return kernels
 
+
+@pytest.mark.parametrize("n,dtype", [(9, "complex128"), (13, "complex128"), (6, "complex128"), (13, "complex64")])
+def test_count_matches_the_graph(n, dtype):
     import torch
-    from torch.profiler import ProfilerActivity, profile
 
     import bench
     from qradient_gb300 import McClean, _lib, tuning
@@ -22,19 +34,20 @@ def test_count_matches_the_profiler(n, dtype):
     c = McClean(n, {"zz": zz}, L, axes=np.zeros((L, n), dtype=int), angles=np.zeros((L, n)), dtype=dtype,
                 grad_mode="history")
     a = torch.zeros(L * n, dtype=torch.float64, device="cuda")
-    c.grad_run_tensors(a)
+    out = (torch.empty(1, dtype=torch.float64, device="cuda"), torch.empty(L * n, dtype=torch.float64, device="cuda"))
+    c.grad_run_tensors(a, out=out)
     torch.cuda.synchronize()
-    for _ in range(2):  # (a process's first profile may come back without kernels)
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            for _ in range(steps):
-                c.grad_run_tensors(a)
-            torch.cuda.synchronize()
-    seen = sum(e.count for e in prof.key_averages() if "qg::" in e.key)
-    if not seen:
-        pytest.skip("the profiler lists no kernels here")
+    try:
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+    except TypeError:
+        pytest.skip("this torch keeps no captured graph")
+    with torch.cuda.graph(g):
+        for _ in range(steps):
+            c.grad_run_tensors(a, out=out)
+    seen = _kernel_nodes(g.raw_cuda_graph())
     lib.qg_profile_enable(1)
     for _ in range(steps):
-        c.grad_run_tensors(a)
+        c.grad_run_tensors(a, out=out)
     torch.cuda.synchronize()
     counted = 0
     for cls in (0, 1, 2):
